@@ -275,9 +275,8 @@ int edgpu_spmv(edgpu_model *m, int storage, int nup, int ndn, const void *x, voi
       Sector_mv<T> v{s->dop<T>(), static_cast<const T *>(x), static_cast<T *>(y), ldx, nvec, s->srs_rows, s->nitems,
                      accumulate != 0};
       MvShape sh = mv_shape<T>(*s);
-      if (s->storage == kSRS && !sh.long_places && s->dn_rows < kSrsVeryLong && (long long)nvec * s->nitems < 304) {
-        // too few items for two per SM: groups of four rows, as many to an item as that leaves
-        v.rows = (int)std::min<long long>(s->srs_rows, std::max<long long>(4, ((long long)nvec * s->up_rows / 304 + 3) / 4 * 4));
+      if (s->storage == kSRS) {
+        v.rows = vec_item_rows(s->srs_rows, s->up_rows, s->dn_rows, s->nitems, nvec);
         v.per = (s->up_rows + v.rows - 1) / v.rows;
       }
       if ((long long)v.per * nvec > INT_MAX) throw ApiError(EDGPU_ERR_ARG, "too many vectors for one call");

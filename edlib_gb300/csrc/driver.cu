@@ -561,11 +561,7 @@ Sector *get_sector(edgpu_model *m, int storage, int nup, int ndn) {
     }
     s->srs_rows = srs_item_rows(s->up_rows, s->dn_rows);
     s->nitems = (s->up_rows + s->srs_rows - 1) / s->srs_rows;
-    if (s->dn_rows < kSrsVeryLong)
-      for (int u0 = 0; u0 < s->up_rows; u0 += s->srs_rows)
-        s->up_hops_item = std::max(s->up_hops_item, up->hrp[std::min(s->up_rows, u0 + s->srs_rows)] - up->hrp[u0]);
-    // short rows with more hops per item than that read them from global memory
-    if (s->dn_rows < kSrsLongRow) s->up_hops_item = std::min(s->up_hops_item, 1024);
+    s->up_hops_item = item_hop_room(s->srs_rows, s->dn_rows, up->kmax);
   } else {
     s->srs_rows = row_item(s->dim);
     s->nitems = (int)((s->dim + s->srs_rows - 1) / s->srs_rows);

@@ -153,6 +153,23 @@ inline int srs_item_rows(int up_rows, int dn_rows) {
   return std::max(1, std::min(r, up_rows));
 }
 
+// SRS rows per item of a product of nvec vectors of one sector (edgpu_spmv): the sector's own, or, where those make too few
+// items for two per SM, as few as that takes, in groups of four.
+inline int vec_item_rows(int srs_rows, int up_rows, int dn_rows, int nitems, long long nvec) {
+  if (dn_rows >= kSrsVeryLong || nvec * nitems >= 304) return srs_rows;
+  return (int)std::min<long long>(srs_rows, std::max<long long>(4, (nvec * up_rows / 304 + 3) / 4 * 4));
+}
+
+// Room in shared memory for the up hops of an item (entries): of any srs_rows consecutive rows, from the longest row,
+// because a product may cut the sector at other rows than multiples of srs_rows (18-site impurity, sector (4,2), two
+// vectors: items of 20 rows with up to 220 hops, where groups of 24 from row 0 on have at most 216).  Tiles read their
+// hops from there alone; short rows with more than 1024 per item read them from global memory.
+inline int item_hop_room(int srs_rows, int dn_rows, int kmax) {
+  if (dn_rows >= kSrsVeryLong) return 0;
+  const int n = srs_rows * kmax;
+  return dn_rows < kSrsLongRow ? std::min(n, 1024) : n;
+}
+
 // Rows per item of a CRS or SOCRS sector: about two items per SM, of 64 to 2048 rows (4900 rows in items of 2048
 // left all but three SMs idle).
 inline int row_item(long long dim) {

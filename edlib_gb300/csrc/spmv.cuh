@@ -913,15 +913,17 @@ __global__ void __launch_bounds__(kMvBlock, MB) k_srs_mv(Src src, int nitems, in
       continue;
     }
     const int Nd = it.Nd;
-    const bool tile = Nd >= kSrsLongRow && Nd < kSrsVeryLong, small = Nd < kSrsLongRow;
+    const bool small = Nd < kSrsLongRow;
+    bool tile = Nd >= kSrsLongRow && Nd < kSrsVeryLong;
     // 16-byte accesses: rows of whole 16-byte pieces on aligned bases
     const bool whole = (Nd * sizeof(T)) % 16 == 0;
     const bool vec = whole && (((uintptr_t)it.x | (uintptr_t)it.dg | (uintptr_t)it.y | (uintptr_t)it.z) & 15) == 0;
     const int nel = it.nrows * Nd;
-    bool near = false;  // short rows: the item's hops fit in shared memory
+    bool near = false;  // the item's hops fit in shared memory; tiles', always (item_hop_room)
     if (tile || small) {
       const int k0 = ldg_t(it.urp), nh = ldg_t(it.urp + it.nrows) - k0;
       near = nh <= hop_cap;
+      tile = tile && near;  // else row by row from global memory
       if (tile)
         for (int q = threadIdx.x; q <= it.nrows; q += kMvBlock) hop_rp[q] = ldg_t(it.urp + q) - k0;
       if (near)

@@ -215,3 +215,33 @@ def test_recurrences_alone_and_in_a_batch_of_many_items(ed):
     alone = [ed.GreensFunction(p, h).compute() for (p, _), h in zip(specs, hams)]
     Gs, _, _ = ed.greens_function_many(specs[0][0], hams)
     assert all(np.array_equal(a, b) for a, b in zip(alone, Gs))
+
+
+# items that lie across the sector's own ones (12 -> 8 rows, 24 -> 20), with more up hops than any of those: the values
+# of a call with many vectors to the last bit, and the oracle's
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("ns,sec,nvec", [(13, (6, 3), 1), (18, (4, 2), 2)])
+def test_items_across_the_sectors_own_ones(ed, precision, ns, sec, nvec):
+    import torch
+    from edlib_gb300 import _abi
+    from oracle.oracle import OracleED
+    params, data = models.random_siam(70 + ns, ns - 1)
+    params.update({"storage.MAX_DIM": 0, "storage.MAX_SIZE": 0})
+    ham = ed.Hamiltonian(ed.Params(params), data, storage="SRS", precision=precision)
+    ham.set_limits(0, 0)
+    n = ham.storage.fill(*sec)
+    ld = (n + 3) // 4 * 4
+    x = torch.randn(40, ld, dtype=torch.float64 if precision == "fp64" else torch.float32, device="cuda")
+    ys = []
+    for k in (nvec, 40):
+        y = torch.zeros_like(x)
+        assert _abi.lib().edgpu_spmv(ham._m, 1, sec[0], sec[1], x.data_ptr(), y.data_ptr(), k, ld,
+                                     _abi.PRECISIONS[precision], 0, torch.cuda.current_stream().cuda_stream) == 0
+        torch.cuda.synchronize()
+        ys.append(y[:nvec, :n])
+    assert torch.equal(ys[0], ys[1])
+    o = OracleED(params, data, "SRS", "SIAM")
+    assert o.fill(*sec) == n
+    w = o.av(x[0, :n].double().cpu().numpy())
+    assert np.abs(ys[0][0].double().cpu().numpy() - w).max() <= TOL[precision] * np.abs(w).max()
+    ham.close()
