@@ -267,7 +267,7 @@ struct EigTask {
   double *hpart2;    // [nchunks][ld] partials of g = V^T V[j]
   double *spart;     // [nsup][2 ld + 2] superchunk sums of s, g and |w|^2 (kCgsSup chunks each)
   double *hv;        // [ld] projection coefficients h = (I - E) s of the step
-  int *ord;          // [ld + 1] update order: [0] columns subtracted exactly, then the column indices; [ld] their number
+  int *ord;          // [ld + 1] update order: [0] columns subtracted exactly, then the column indices
   int *cnt;          // [nsup + 1] arrival counters of the dot reduction, zero between launches
   double *npart;     // [2][nchunks] |w|^2 before and after the projection
   double *E;         // ld x ld Gram deviation V^T V - I of the basis (column-major)
