@@ -626,7 +626,7 @@ int edgpu_bench_cgs(edgpu_model *m, int storage, int nup, int ndn, int nbasis, i
       const long long n = s->dim, ldv = (n + 16 / (long long)sizeof(T) - 1) / (16 / (long long)sizeof(T)) *
                                               (16 / (long long)sizeof(T));
       const int ld = nbasis + 1;
-      const int nch = (int)((n + cgs_chunk<T>(n) - 1) / cgs_chunk<T>(n));
+      const int nch = (int)((n + kCgsChunk - 1) / kCgsChunk);
       // ntasks independent bases of the sector: nbasis columns (+1 spare), w, a saved copy of w
       DBuf V(c->alloc, sizeof(T) * (size_t)ntasks * (nbasis + 1) * ldv), W(c->alloc, sizeof(T) * (size_t)ntasks * ldv),
           W0(c->alloc, sizeof(T) * (size_t)ntasks * ldv),
@@ -653,7 +653,6 @@ int edgpu_bench_cgs(edgpu_model *m, int storage, int nup, int ndn, int nbasis, i
         t.op = s->dop<T>();
         t.chunk_begin = (int)cmap.size();
         t.nchunks = nch;
-        t.chunk = cgs_chunk<T>(n);
         t.n = n;
         t.ldv = ldv;
         t.m = nbasis;

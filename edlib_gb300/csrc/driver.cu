@@ -750,7 +750,7 @@ class EigBatch {
     size_t nvec = 0, nsmall = 0;
     for (auto *j : jobs) {
       const long long n = j->s->dim, ldv = padded_ld<T>(n);
-      const size_t nch = (size_t)((n + cgs_chunk<T>(n) - 1) / cgs_chunk<T>(n));
+      const size_t nch = (size_t)((n + kCgsChunk - 1) / kCgsChunk);
       const size_t gp = (size_t)(j->m + 1) * (j->m + 2) / 2;
       nvec += 2 * al((sizeof(T) * (size_t)(j->m + 1) * ldv + 7) / 8) + al((sizeof(T) * (size_t)ldv + 7) / 8);
       const size_t nsup = (size_t)cgs_nsup((int)nch);
@@ -772,7 +772,7 @@ class EigBatch {
     for (size_t i = 0; i < jobs.size(); ++i) {
       EigSectorJob *j = jobs[i];
       const long long n = j->s->dim, ldv = padded_ld<T>(n);
-      const size_t nch = (size_t)((n + cgs_chunk<T>(n) - 1) / cgs_chunk<T>(n));
+      const size_t nch = (size_t)((n + kCgsChunk - 1) / kCgsChunk);
       const size_t gp = (size_t)(j->m + 1) * (j->m + 2) / 2;
       const size_t vb = al((sizeof(T) * (size_t)(j->m + 1) * ldv + 7) / 8);
       Slot sl;
@@ -1049,7 +1049,7 @@ class EigBatch {
       const Slot &sl = slots_[i];
       const Sector &s = *sl.job->s;
       const long long n = s.dim;
-      const int nch = (int)((n + cgs_chunk<T>(n) - 1) / cgs_chunk<T>(n));
+      const int nch = (int)((n + kCgsChunk - 1) / kCgsChunk);
       EigTask<T> &t = tasks_[i];
       t.op = s.dop<T>();
       t.srs_rows = s.srs_rows;
@@ -1057,7 +1057,6 @@ class EigBatch {
       t.nitems = s.nitems;
       t.chunk_begin = (int)chunk_task.size();
       t.nchunks = nch;
-      t.chunk = cgs_chunk<T>(n);
       t.n = n;
       t.ldv = padded_ld<T>(n);
       t.m = sl.job->m;

@@ -227,19 +227,11 @@ struct LzTask {
 #ifndef EDGPU_CGS_MIN_BLOCKS
 #define EDGPU_CGS_MIN_BLOCKS 2
 #endif
-// Vector elements per Gram-Schmidt chunk, from the vector's length alone (so that a sector's sums do not depend on
-// its batch).  FP32 passes stream at the memory rate from 4096 on.  FP64 ones are bound by FP64 issue (two lanes per
-// clock and SM): a chunk is one SM's work, and 65,536 states in chunks of 4096 kept a block busy 0.5 ms per restart
-// with most SMs idle, so short vectors take 512 and long ones 2048 (smaller ones spend more on the warp sums: 28 % of
-// the multiply-adds at 1024, 14 % at 2048).
-template <typename T>
-constexpr int kCgsBig = sizeof(T) == 4 ? 4096 : 2048;
-template <typename T>
-constexpr int kCgsSmall = sizeof(T) == 4 ? 4096 : 512;
-template <typename T>
-__host__ __device__ inline int cgs_chunk(long long n) {
-  return n <= 65536 ? kCgsSmall<T> : kCgsBig<T>;
-}
+// Vector elements per Gram-Schmidt chunk, in every precision: sums over a vector are formed chunk by chunk, so the length
+// is part of the values (FP64 chunks of 512 or 2048, shorter by the vector's length, gave other last bits).  FP64 passes
+// are bound by FP64 issue (two lanes per clock and SM) and a chunk is one SM's work, so where chunks are few the dot pass
+// divides a chunk's columns and the restart its elements among blocks (krylov.cu: dot_parts, launch_eig_restart).
+constexpr int kCgsChunk = 4096;
 constexpr int kCgsSup = 64;                  // chunks per split of the dot pass's partials reduction
 __host__ __device__ inline int cgs_nsup(int nchunks) { return (nchunks + kCgsSup - 1) / kCgsSup; }
 constexpr int kMaxLd = 128;      // largest projected-matrix dimension (ncv + 1)
@@ -254,8 +246,7 @@ struct EigTask {
   int item_begin;
   int nitems;
   int chunk_begin;   // first entry of this task in the chunk map
-  int nchunks;       // ceil(n / chunk)
-  int chunk;         // cgs_chunk<T>(n)
+  int nchunks;       // ceil(n / kCgsChunk)
   long long n;
   long long ldv;     // column stride of V (n rounded up to 16 bytes)
   int m;             // basis vectors before a restart (ncv, clamped to n)
