@@ -202,8 +202,7 @@ struct MvTask {
   double c;
 };
 
-// Plain Lanczos recurrence (include/edlib/Lanczos.h:36-77) over rotating buffers.  The buffers hold unnormalised
-// vectors u: v = u r with r = scal[2] (1 for the normalised start vector), so that no pass only scales one.
+// Plain Lanczos recurrence (include/edlib/Lanczos.h:36-77) over rotating buffers.
 template <typename T>
 struct LzTask {
   const SectorOp<T> *op;
@@ -215,7 +214,7 @@ struct LzTask {
   double *beta;       // [nlanc + 1]
   double *part_a;     // [nitems]
   double *part_b;     // [nitems]
-  double *scal;       // [0] alf, [1] bet, [2] r = 1 / bet of the current vector, [3] r of the one before
+  double *scal;       // [0] alf, [1] bet
   int *state;         // [0] done, [1] nlanc, [2] items of the operator done in this step, [3] of the alpha pass
   int nlanc_max;
 };

@@ -138,9 +138,6 @@ void trace_coefficients(const std::vector<LzJob<T> *> &jobs, int nlanc, const ch
   }
 }
 
-// LzTask::scal of a normalised start vector
-static const double kLzScal0[4] = {0.0, 0.0, 1.0, 1.0};
-
 // The recurrences of FP64 jobs in float-float (`ff`, the mixed mode on spin-resolved sectors): each job's
 // normalised FP64 start vector is rewritten in place as float-float (the same 8 bytes per element), the three
 // buffers are read as float-float, and the steps run on the sector's float-float tables; alpha / beta stay FP64.
@@ -158,11 +155,11 @@ void run_lanczos_ff(edgpu_model *m, std::vector<LzJob<double> *> &jobs, int nlan
     J.beta = DBuf(c->alloc, sizeof(double) * (nlanc + 1));
     J.part_a = DBuf(c->alloc, sizeof(double) * s.nitems);
     J.part_b = DBuf(c->alloc, sizeof(double) * s.nitems);
-    J.scal = DBuf(c->alloc, sizeof(double) * 4);
+    J.scal = DBuf(c->alloc, sizeof(double) * 2);
     J.state = DBuf(c->alloc, sizeof(int) * 4);
     CK(cudaMemsetAsync(J.alpha.p, 0, sizeof(double) * nlanc, c->stream));
     CK(cudaMemsetAsync(J.beta.p, 0, sizeof(double) * (nlanc + 1), c->stream));
-    CK(cudaMemcpyAsync(J.scal.p, kLzScal0, sizeof(kLzScal0), cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemsetAsync(J.scal.p, 0, sizeof(double) * 2, c->stream));
     CK(cudaMemsetAsync(J.state.p, 0, sizeof(int) * 4, c->stream));
     LzTask<ffloat> &t = tasks[q];
     t.op = s.dop<ffloat>();
@@ -216,11 +213,11 @@ void run_lanczos(edgpu_model *m, std::vector<LzJob<T> *> &jobs, int nlanc, bool 
     J.beta = DBuf(c->alloc, sizeof(double) * (nlanc + 1));
     J.part_a = DBuf(c->alloc, sizeof(double) * s.nitems);
     J.part_b = DBuf(c->alloc, sizeof(double) * s.nitems);
-    J.scal = DBuf(c->alloc, sizeof(double) * 4);
+    J.scal = DBuf(c->alloc, sizeof(double) * 2);
     J.state = DBuf(c->alloc, sizeof(int) * 4);
     CK(cudaMemsetAsync(J.alpha.p, 0, sizeof(double) * nlanc, c->stream));
     CK(cudaMemsetAsync(J.beta.p, 0, sizeof(double) * (nlanc + 1), c->stream));
-    CK(cudaMemcpyAsync(J.scal.p, kLzScal0, sizeof(kLzScal0), cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemsetAsync(J.scal.p, 0, sizeof(double) * 2, c->stream));
     CK(cudaMemsetAsync(J.state.p, 0, sizeof(int) * 4, c->stream));
     LzTask<T> &t = tasks[q];
     t.op = s.dop<T>();

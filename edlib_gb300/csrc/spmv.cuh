@@ -165,13 +165,13 @@ struct SrsItem {
   const Hop<T> *uh;
   double *dot;               // the item's part of <x, y>, or null
   const LzTask<T> *lz;       // the recurrence it belongs to (with dot)
-  T c, r;                    // y = r (H x + c z)
+  T c;                       // y = H x + c z
   int Nd, ld, u0, nrows, vloc, skip;
 };
 
 template <typename T>
 __device__ __forceinline__ void fetch_item(SrsItem<T> &d, const SectorOp<T> *opp, int srs_rows, int li, const T *x, T *y,
-                                           const T *z, T c, T r, const LzTask<T> *lz) {
+                                           const T *z, T c, const LzTask<T> *lz) {
   const SectorOp<T> &op = *opp;
   const int Nd = op.dn_rows, u0 = li * srs_rows;
   const long long lo = (long long)u0 * Nd;
@@ -189,7 +189,6 @@ __device__ __forceinline__ void fetch_item(SrsItem<T> &d, const SectorOp<T> *opp
   d.dot = lz ? lz->part_a + li : nullptr;
   d.lz = lz;
   d.c = c;
-  d.r = r;
   d.Nd = Nd;
   d.ld = op.dn_ld;
   d.u0 = u0;
@@ -462,10 +461,6 @@ __device__ __forceinline__ void srs_tile(const SrsItem<T> &it, const ItemHops<T>
 #pragma unroll
       for (int cc = 0; cc < C; ++cc) a[r][cc] = p.v[cc];
     }
-    if (MD) {
-#pragma unroll
-      for (int cc = 0; cc < C; ++cc) a[r][cc] = it.r * a[r][cc];
-    }
     T *__restrict__ y = it.y + row(r);
     if constexpr (VEC) {
       if (mine) store_lanes(y, a[r]);
@@ -621,10 +616,6 @@ __device__ __noinline__ DotAcc srs_longrow(const SrsItem<T> &it, const T *__rest
 #pragma unroll
         for (int cc = 0; cc < C; ++cc) a[cc] = p.v[cc];
       }
-      if (MD) {
-#pragma unroll
-        for (int cc = 0; cc < C; ++cc) a[cc] = it.r * a[cc];
-      }
 #pragma unroll
       for (int cc = 0; cc < C; ++cc) {
         if (cc < nc) {
@@ -723,7 +714,6 @@ __device__ __noinline__ DotAcc srs_short(const SrsItem<T> &it, const ItemHops<T>
 #pragma unroll
     for (int r = 0; r < RI; ++r) {
       if (r >= nr) continue;
-      if (MD) a[r] = it.r * a[r];
       it.y[ro[r]] = renorm(a[r]);
       if (MD && it.dot) dot_add(acc, own.v[r], a[r]);
     }
@@ -742,7 +732,7 @@ __device__ __forceinline__ T row_sum(T v) {
   return v;
 }
 
-// One item of a sector (CRS, SOCRS): y[lo:hi) = r ((H x)[lo:hi) + c z[lo:hi)); the thread's part of <x, y>.  L lanes share
+// One item of a sector (CRS, SOCRS): y[lo:hi) = (H x)[lo:hi) + c z[lo:hi); the thread's part of <x, y>.  L lanes share
 // a row and add their parts by a fixed butterfly.  CRS: lane q takes the row's entries q, q + L, ..., so that a row's
 // values and columns are read side by side and its x loads are in flight at once; with one thread per row each waited
 // for its own chain of loads (4900 rows of 17 entries, one FP64 vector: 27 -> 7 us cold).  SOCRS: lane q takes
@@ -750,7 +740,7 @@ __device__ __forceinline__ T row_sum(T v) {
 // 91 -> 38 us, the rows' own 64-bit decoding of every transition before).
 template <typename T, int ST>
 __device__ __forceinline__ DotAcc mv_item(const SectorOp<T> *opp, int rows, long long li, const T *__restrict__ x,
-                                          T *__restrict__ y, const T *z, T c, T r, bool want_dot) {
+                                          T *__restrict__ y, const T *z, T c, bool want_dot) {
   constexpr int L = ST == kCRS ? 4 : 8;
   const SectorOp<T> &op = *opp;
   long long lo, hi;
@@ -786,7 +776,6 @@ __device__ __forceinline__ DotAcc mv_item(const SectorOp<T> *opp, int rows, long
     if (in && q == 0) {
       if constexpr (ST == kSOCRS) v += ldg_t(op.diag + i) * x[i];
       if (z) v = v + c * z[i];
-      v = r * v;
       y[i] = v;
       if (want_dot) dot_add(acc, x[i], v);
     }
@@ -796,20 +785,16 @@ __device__ __forceinline__ DotAcc mv_item(const SectorOp<T> *opp, int rows, long
 
 // <x, y> of an item into its recurrence's parts; the block that finishes the task's last item sums them: alf.
 template <typename T, int NT>
-__device__ __forceinline__ void emit_dot(const LzTask<T> &t, DotAcc &acc, double r, double *dst, double *red) {
+__device__ __forceinline__ void emit_dot(const LzTask<T> &t, DotAcc &acc, double *dst, double *red) {
   const double s = block_sum<NT>(dot_value(acc), red);
-  if (threadIdx.x == 0) *dst = s * r;
+  if (threadIdx.x == 0) *dst = s;
   double alf;
   if (last_block_sum<NT>(t.part_a, t.nitems, t.state + 2, red, alf) && threadIdx.x == 0) t.scal[0] = alf;
 }
-// r as FP64, as the vectors' type holds it
-__device__ __forceinline__ double as_double(float r) { return r; }
-__device__ __forceinline__ double as_double(double r) { return r; }
-__device__ __forceinline__ double as_double(ffloat r) { return ff_value(r); }
 
 // ---------------------------------------------------------------- where an operator launch's items come from
-// get(it, f): f(op, srs_rows, li, x, y, z, c, r, lz) for item it: y = r (H x + c z), <x, y> r into lz's parts where lz
-// is given; or false where its task has nothing to do.  kEarly: its launches may be launch_pdl's.
+// get(it, f): f(op, srs_rows, li, x, y, z, c, lz) for item it: y = H x + c z, <x, y> into lz's parts where lz is given, or
+// false where its task has nothing to do.  kEarly: its launches may be launch_pdl's.
 
 // generic batch: y = H x (+ c z)
 template <typename T>
@@ -821,7 +806,7 @@ struct MvSource {
   __device__ __forceinline__ bool get(int it, F &&f) const {
     const MvTask<T> &t = tasks[item_task[it]];
     const int li = it - t.item_begin;
-    f(t.op, t.srs_rows, li, t.x, t.y, t.z, (T)t.c, T(1), (const LzTask<T> *)nullptr);
+    f(t.op, t.srs_rows, li, t.x, t.y, t.z, (T)t.c, (const LzTask<T> *)nullptr);
     return true;
   }
 };
@@ -840,14 +825,13 @@ struct VecSource {
   __device__ __forceinline__ bool get(int it, F &&f) const {
     const int q = it / per;
     T *yq = y + q * ld;
-    f(op, rows, it - q * per, x + q * ld, yq, acc ? yq : nullptr, T(1), T(1), (const LzTask<T> *)nullptr);
+    f(op, rows, it - q * per, x + q * ld, yq, acc ? yq : nullptr, T(1), (const LzTask<T> *)nullptr);
     return true;
   }
 };
 
-// Lanczos recurrence, phase 1.  Iteration iter (0-based) of Lanczos.h:44-68 on unnormalised vectors: with v = u r,
-// w = H v - bet v_prev = r (H u - bet^2 r_prev u_prev), u = buf[iter % 3], w = buf[(iter + 1) % 3],
-// u_prev = buf[(iter + 2) % 3]; a finished recurrence has nothing to do.
+// Lanczos recurrence, phase 1.  Iteration iter (0-based) of Lanczos.h:44-68: v = buf[iter % 3],
+// w = buf[(iter + 1) % 3] = H v - bet buf[(iter + 2) % 3]; a finished recurrence has nothing to do.
 template <typename T>
 struct LzSource {
   static constexpr bool kEarly = true;
@@ -858,9 +842,8 @@ struct LzSource {
   __device__ __forceinline__ bool get(int it, F &&f) const {
     const LzTask<T> &t = tasks[item_task[it]];
     if (t.state[0]) return false;
-    const double bet = t.scal[1];
     f(t.op, t.srs_rows, it - t.item_begin, t.buf[iter % 3], t.buf[(iter + 1) % 3],
-      iter == 0 ? nullptr : t.buf[(iter + 2) % 3], (T)(-bet * bet * t.scal[3]), (T)t.scal[2], &t);
+      iter == 0 ? nullptr : t.buf[(iter + 2) % 3], (T)(-t.scal[1]), &t);
     return true;
   }
 };
@@ -878,7 +861,7 @@ struct EigSource {
     const EigTask<T> &t = tasks[item_task[it]];
     if (!probe_y && (t.st[2] || t.st[1] != 0)) return false;  // full, or orthogonalising a random vector
     f(t.op, t.srs_rows, it - t.item_begin, probe_y ? t.V : t.V + (long long)t.st[0] * t.ldv, probe_y ? probe_y : t.w,
-      (const T *)nullptr, T(0), T(1), (const LzTask<T> *)nullptr);
+      (const T *)nullptr, T(0), (const LzTask<T> *)nullptr);
     return true;
   }
 };
@@ -895,8 +878,8 @@ __global__ void __launch_bounds__(kMvBlock, MB) k_srs_mv(Src src, int nitems, in
   const ItemHops<T> hops{reinterpret_cast<Hop<T> *>(smem_raw + align16(sizeof(T) * (size_t)xs_cap)), hop_rp};
   // items from the last on: the batches list their sectors by size, and the largest items first leave the shortest tail
   auto fetch = [&](int i, SrsItem<T> &d) {
-    if (i < nitems && !src.get(nitems - 1 - i, [&](const SectorOp<T> *op, int srs_rows, int li, const T *x, T *y, const T *z, T c, T r, const LzTask<T> *lz) {
-          fetch_item<T>(d, op, srs_rows, li, x, y, MZ ? z : nullptr, c, r, MD ? lz : nullptr);
+    if (i < nitems && !src.get(nitems - 1 - i, [&](const SectorOp<T> *op, int srs_rows, int li, const T *x, T *y, const T *z, T c, const LzTask<T> *lz) {
+          fetch_item<T>(d, op, srs_rows, li, x, y, MZ ? z : nullptr, c, MD ? lz : nullptr);
         }))
       d.skip = 1;
   };
@@ -956,7 +939,7 @@ __global__ void __launch_bounds__(kMvBlock, MB) k_srs_mv(Src src, int nitems, in
     } else {
       acc = srs_longrow<T, MZ, MD>(it, nel <= xs_cap ? xs : it.xi);
     }
-    if (MD && it.dot) emit_dot<T, kMvBlock>(*it.lz, acc, as_double(it.r), it.dot, red);
+    if (MD && it.dot) emit_dot<T, kMvBlock>(*it.lz, acc, it.dot, red);
     __syncthreads();  // xs and items[p] are free, items[p ^ 1] is there
   }
 }
@@ -1048,8 +1031,8 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_srs_long(Src src, int nitems)
   for (int i = blockIdx.x; i < nitems; i += gridDim.x) {
     __syncthreads();  // the previous item is no longer read
     if (threadIdx.x == 0) {
-      it.skip = !src.get(i, [&](const SectorOp<T> *op, int srs_rows, int li, const T *x, T *y, const T *z, T c, T r, const LzTask<T> *lz) {
-        fetch_item<T>(it, op, srs_rows, li, x, y, MZ ? z : nullptr, c, r, MD ? lz : nullptr);
+      it.skip = !src.get(i, [&](const SectorOp<T> *op, int srs_rows, int li, const T *x, T *y, const T *z, T c, const LzTask<T> *lz) {
+        fetch_item<T>(it, op, srs_rows, li, x, y, MZ ? z : nullptr, c, MD ? lz : nullptr);
       }) || !it.skip;
     }
     __syncthreads();
@@ -1124,10 +1107,6 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_srs_long(Src src, int nitems)
 #pragma unroll
               for (int r = 0; r < RI; ++r) a[r] = p.v[r];
             }
-            if (MD) {
-#pragma unroll
-              for (int r = 0; r < RI; ++r) a[r] = it.r * a[r];
-            }
             st_cols<T>(yr, a, nc, whole);
             if (MD && it.dot) {
               const Lanes<T> q = xs[u];
@@ -1138,7 +1117,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_srs_long(Src src, int nitems)
           }
         }
       }
-      if (MD && it.dot) emit_dot<T, NT>(*it.lz, acc, as_double(it.r), it.dot, red);
+      if (MD && it.dot) emit_dot<T, NT>(*it.lz, acc, it.dot, red);
     }
   }
 }
@@ -1149,9 +1128,9 @@ __global__ void __launch_bounds__(kMvBlock, 3) k_row_mv(Src src, int nitems) {
   __shared__ double red[kMvBlock / 32];
   if constexpr (Src::kEarly) pdl_enter();
   for (int i = blockIdx.x; i < nitems; i += gridDim.x)
-    src.get(i, [&](const SectorOp<T> *op, int rows, int li, const T *x, T *y, const T *z, T c, T r, const LzTask<T> *lz) {
-      DotAcc acc = mv_item<T, ST>(op, rows, li, x, y, z, c, r, lz != nullptr);
-      if (lz) emit_dot<T, kMvBlock>(*lz, acc, as_double(r), lz->part_a + li, red);
+    src.get(i, [&](const SectorOp<T> *op, int rows, int li, const T *x, T *y, const T *z, T c, const LzTask<T> *lz) {
+      DotAcc acc = mv_item<T, ST>(op, rows, li, x, y, z, c, lz != nullptr);
+      if (lz) emit_dot<T, kMvBlock>(*lz, acc, lz->part_a + li, red);
     });
 }
 
