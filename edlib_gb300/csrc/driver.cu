@@ -300,23 +300,11 @@ SpinCsr *get_spin(edgpu_model *m, int spin, int k) {
   launch_pack_hops<double>(s->col.as<int>(), s->v64.as<double>(), s->nnz, s->uh64.as<Hop<double>>(), c->stream);
   launch_pack_hops<float>(s->col.as<int>(), s->v32.as<float>(), s->nnz, s->uh32.as<Hop<float>>(), c->stream);
   if (spin == 1 && rows >= kSrsLongRow && rows < kSrsVeryLong) {
-    const int km = std::max(1, s->kmax);
-    const size_t cells = (size_t)km * s->ld;
+    const int cells = std::max(1, s->kmax) * s->ld;
     s->slot4 = DBuf(c->alloc, sizeof(unsigned short) * cells);
     s->slot2 = DBuf(c->alloc, sizeof(unsigned short) * cells);
-    s->sv64 = DBuf(c->alloc, sizeof(double) * cells);
-    s->sv32 = DBuf(c->alloc, sizeof(float) * cells);
-    s->tlen4 = DBuf(c->alloc, sizeof(int) * s->ld);
-    s->tlen2 = DBuf(c->alloc, sizeof(int) * s->ld);
-    DBuf order4(c->alloc, sizeof(short) * cells), order2(c->alloc, sizeof(short) * cells);
-    for (DBuf *o : {&order4, &order2}) CK(cudaMemsetAsync(o->p, 0xff, sizeof(short) * cells, c->stream));
-    for (DBuf *o : {&s->slot4, &s->slot2}) CK(cudaMemsetAsync(o->p, 0, sizeof(unsigned short) * cells, c->stream));
-    launch_tile_schedule(s->ell_col.as<int>(), s->len.as<int>(), (int)rows, s->ld, km, 4, s->slot4.as<unsigned short>(),
-                         order4.as<short>(), s->tlen4.as<int>(), c->stream);
-    launch_tile_schedule(s->ell_col.as<int>(), s->len.as<int>(), (int)rows, s->ld, km, 2, s->slot2.as<unsigned short>(),
-                         order2.as<short>(), s->tlen2.as<int>(), c->stream);
-    launch_order_values<float>(s->ell_v32.as<float>(), order4.as<short>(), s->ld, km, s->sv32.as<float>(), c->stream);
-    launch_order_values<double>(s->ell_v64.as<double>(), order2.as<short>(), s->ld, km, s->sv64.as<double>(), c->stream);
+    launch_tile_slots(s->ell_col.as<int>(), cells, (int)rows, 4, s->slot4.as<unsigned short>(), c->stream);
+    launch_tile_slots(s->ell_col.as<int>(), cells, (int)rows, 2, s->slot2.as<unsigned short>(), c->stream);
   }
   const DevVProd &vp = m->vprod.dev;
   if (vp.nW > 0 && spin == 0) {
@@ -355,7 +343,7 @@ static void ensure_long(edgpu_model *m, SpinCsr *s) {
   CK(cudaMemsetAsync(order.p, 0xff, sizeof(short) * cells, c->stream));
   CK(cudaMemsetAsync(s->slot1.p, 0, sizeof(unsigned short) * cells, c->stream));
   s->tlen1 = DBuf(c->alloc, sizeof(int) * s->ld);
-  launch_tile_schedule(s->ell_col.as<int>(), s->len.as<int>(), s->rows, s->ld, km, 1, s->slot1.as<unsigned short>(),
+  launch_long_schedule(s->ell_col.as<int>(), s->len.as<int>(), s->rows, s->ld, km, s->slot1.as<unsigned short>(),
                        order.as<short>(), s->tlen1.as<int>(), c->stream);
   launch_order_values<float>(s->ell_v32.as<float>(), order.as<short>(), s->ld, km, s->lv32.as<float>(), c->stream);
   launch_order_values<double>(s->ell_v64.as<double>(), order.as<short>(), s->ld, km, s->lv64.as<double>(), c->stream);
@@ -419,7 +407,6 @@ void ensure_ff(edgpu_model *m, Sector *s) {
       launch_pack_hops<ffloat>(sp->col.as<int>(), sp->vff.as<ffloat>(), sp->nnz, sp->uhff.as<Hop<ffloat>>(), c->stream);
     }
     if (sp->lv64.p && !sp->lvff.p) conv(sp->lvff, sp->lv64, (long long)std::max(1, sp->kmax) * sp->ld);
-    if (sp->sv64.p && !sp->svff.p) conv(sp->svff, sp->sv64, (long long)std::max(1, sp->kmax) * sp->ld);
     if (sp->vd_cells && !sp->vd_vff.p) conv(sp->vd_vff, sp->vd_v64, sp->vd_cells);
   }
   conv(s->diagff, s->diag64, s->dim);
@@ -447,8 +434,6 @@ void ensure_ff(edgpu_model *m, Sector *s) {
   o.dn_ld = d.dn_ld;
   o.up_hop = up->uhff.as<Hop<ffloat>>();
   o.dn_slot = d.dn_slot;
-  o.dn_sval = dn->svff.as<ffloat>();
-  o.dn_tlen = d.dn_tlen;
   SpinCsr *both[2] = {up, dn};
   for (int q = 0; q < 2; ++q) {
     o.long_slot[q] = d.long_slot[q];
@@ -530,10 +515,6 @@ Sector *get_sector(edgpu_model *m, int storage, int nup, int ndn) {
     s->op32.up_hop = up->uh32.as<Hop<float>>();
     s->op64.dn_slot = dn->slot2.as<unsigned short>();
     s->op32.dn_slot = dn->slot4.as<unsigned short>();
-    s->op64.dn_sval = dn->sv64.as<double>();
-    s->op64.dn_tlen = dn->tlen2.as<int>();
-    s->op32.dn_tlen = dn->tlen4.as<int>();
-    s->op32.dn_sval = dn->sv32.as<float>();
     s->op64.nV = s->op32.nV = (int)m->Vs.size();
     s->op64.V_ = s->op32.V_ = m->dVs.as<Transition>();
     s->op64.V_val = m->dVsv64.as<double>();
@@ -561,11 +542,13 @@ Sector *get_sector(edgpu_model *m, int storage, int nup, int ndn) {
     }
     s->srs_rows = srs_item_rows(s->up_rows, s->dn_rows);
     s->nitems = (s->up_rows + s->srs_rows - 1) / s->srs_rows;
-    s->up_hops_item = item_hop_room(s->srs_rows, s->dn_rows, up->kmax);
+    s->up_kmax = up->kmax;
   } else {
     s->srs_rows = row_item(s->dim);
     s->nitems = (int)((s->dim + s->srs_rows - 1) / s->srs_rows);
   }
+  s->lz_rows = lz_item_rows(storage, s->up_rows, s->dn_rows);
+  s->lz_nitems = (int)(((storage == kSRS ? s->up_rows : s->dim) + s->lz_rows - 1) / s->lz_rows);
   if (storage == kCRS) {
     DBuf count(c->alloc, sizeof(long long) * s->dim), tmp(c->alloc, sizeof(long long) * scan_tmp_size(s->dim)),
         err(c->alloc, sizeof(int));
@@ -608,20 +591,21 @@ Sector *get_sector(edgpu_model *m, int storage, int nup, int ndn) {
   return raw;
 }
 
-// shared memory an operator launch over this sector needs (see spmv.cuh)
+// shared memory an operator launch over this sector needs (see spmv.cuh); lz: with a recurrence's items
 template <typename T>
-MvShape mv_shape(const Sector &s) {
+MvShape mv_shape(const Sector &s, bool lz) {
   MvShape sh{s.storage, 0};
   if (s.storage == kSRS) {
     // interleaved rows are read in whole groups of four, also where an item has fewer
-    const long long rows = s.dn_rows < kSrsVeryLong ? (s.srs_rows + 3) / 4 * 4 : s.srs_rows;
+    const int item = lz ? s.lz_rows : s.srs_rows;
+    const long long rows = s.dn_rows < kSrsVeryLong ? (item + 3) / 4 * 4 : item;
     const long long cap = (long long)(120 * 1024) / (long long)sizeof(T);
     if (srs_two_pass(s.up_rows, s.dn_rows)) {
       sh.long_places = std::max(s.up_rows, s.dn_rows);
     } else {
       sh.other = 1;
       sh.xs_elems = (int)(s.dn_rows < kSrsVeryLong ? rows * s.dn_rows : std::min(rows * s.dn_rows, cap));
-      sh.hop_elems = s.up_hops_item;
+      sh.hop_elems = item_hop_room(item, s.dn_rows, s.up_kmax);
     }
   }
   return sh;
@@ -1732,8 +1716,8 @@ int diag_many_dispatch(edgpu_model *const *ms, int count, const edgpu_diag_param
   return diag_many_impl<double>(ms, count, p, npairs);
 }
 
-template MvShape mv_shape<float>(const Sector &);
-template MvShape mv_shape<double>(const Sector &);
+template MvShape mv_shape<float>(const Sector &, bool);
+template MvShape mv_shape<double>(const Sector &, bool);
 
 template void apply_h<float>(edgpu_model *, Sector *, const float *, float *, const float *, double);
 template void apply_h<double>(edgpu_model *, Sector *, const double *, double *, const double *, double);

@@ -214,14 +214,11 @@ struct SectorOp {
   const int *dn_len, *dn_ell_col;
   const T *dn_ell_val;
   int dn_ld;
-  // the up-spin CSR with source row and value side by side; the k-major down-spin matrix with columns by their
-  // tile_slot and each row's entries in the tiles' order (k_tile_schedule; rows of kSrsLongRow to kSrsVeryLong - 1
-  // states), fillers with value 0
+  // the up-spin CSR with source row and value side by side; the columns of dn_ell_col by their tile_slot (rows of
+  // kSrsLongRow to kSrsVeryLong - 1 states)
   const Hop<T> *up_hop;
   const unsigned short *dn_slot;
-  const T *dn_sval;
-  const int *dn_tlen;  // entries to walk per row, fillers among them
-  // two-pass sectors: the up [0] and down [1] matrices k-major in the order of k_tile_schedule for one column per lane
+  // two-pass sectors: the up [0] and down [1] matrices k-major in the order of k_long_schedule
   const unsigned short *long_slot[2];
   const T *long_val[2];
   const int *long_len[2];

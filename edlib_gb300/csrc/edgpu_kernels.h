@@ -99,11 +99,13 @@ void launch_vprod_dn(const DevModel &m, const DevVProd &vp, int k, int rows, int
 // (column, value) pairs of n table entries
 template <typename T>
 void launch_pack_hops(const int *col, const T *val, long long n, Hop<T> *out, cudaStream_t st);
-// The k-major matrix of a spin in the tiles' order for C columns per lane (see k_tile_schedule): order[k * ld + d] = the
-// entry of row d taken as its k-th, or -1 for a filler, slot the tile_slot position it reads, and tlen[d] how many
-// entries, fillers among them, row d has.
-void launch_tile_schedule(const int *ell_col, const int *len, int rows, int ld, int kmax, int C, unsigned short *slot,
-                          short *order, int *tlen, cudaStream_t st);
+// slot[i] = tile_slot of column ell_col[i], for tiles of C columns per lane
+void launch_tile_slots(const int *ell_col, int n, int rows, int C, unsigned short *slot, cudaStream_t st);
+// The k-major matrix of a spin in the order of the two-pass kernels (see k_long_schedule): order[k * ld + d] = the entry
+// of row d taken as its k-th, or -1 for a filler, slot the column it reads, and tlen[d] how many entries, fillers among
+// them, row d has.
+void launch_long_schedule(const int *ell_col, const int *len, int rows, int ld, int kmax, unsigned short *slot, short *order,
+                          int *tlen, cudaStream_t st);
 // out[k * ld + d] = val[order[k * ld + d] * ld + d], 0 for fillers
 template <typename T>
 void launch_order_values(const T *val, const short *order, int ld, int kmax, T *out, cudaStream_t st);
@@ -134,13 +136,17 @@ __host__ __device__ inline bool srs_two_pass(int up_rows, int dn_rows) {
 // shared memory; rows longer than 6144 elements one or a few per item); short rows take about kItemElems
 // elements per item.  Measured on Anderson-12 (FP32 eigen-solve of all sectors): 0.575 s with 4096, 0.531 s
 // with 8192, 0.543 s with 16384, 0.595 s with 2048 elements per item.
-inline int srs_item_rows(int up_rows, int dn_rows) {
-  if (srs_two_pass(up_rows, dn_rows)) return kLongRows;
+inline int srs_item_elems() {
   static const int target = [] {  // elements per item of long rows (EDGPU_SRS_ITEM_ELEMS, for measurements)
     const char *e = getenv("EDGPU_SRS_ITEM_ELEMS");
     const int v = e ? atoi(e) : 0;
     return v >= 512 && v <= 24576 ? v : 8192;  // 8192: 8 % less eigen-solve time than 4096 on Anderson-12
   }();
+  return target;
+}
+inline int srs_item_rows(int up_rows, int dn_rows) {
+  if (srs_two_pass(up_rows, dn_rows)) return kLongRows;
+  const int target = srs_item_elems();
   int r;
   if (dn_rows >= kSrsLongRow && dn_rows < kSrsVeryLong) r = std::max(4, std::min(24576 / dn_rows, target / dn_rows) & ~3);
   else if (dn_rows >= kSrsLongRow) r = std::max(1, 24576 / dn_rows);  // very long rows: as many as stage in 96 KB
@@ -150,6 +156,16 @@ inline int srs_item_rows(int up_rows, int dn_rows) {
   // sectors of too few rows for an item per SM of that size: about one item per SM, of at least four rows
   if (dn_rows >= kSrsLongRow && dn_rows < kSrsVeryLong)
     r = std::min({r, kTileRows, std::max(4, ((up_rows + 151) / 152 + 3) & ~3)});
+  return std::max(1, std::min(r, up_rows));
+}
+
+// Rows per item of a recurrence.  Its sums are formed item by item, so the item size is part of the values: not by the
+// number of SMs or the storage's needs, as srs_item_rows and row_item, but from the row length alone.
+inline int lz_item_rows(int storage, int up_rows, int dn_rows) {
+  if (storage != kSRS) return kItemElems;
+  if (dn_rows >= kSrsVeryLong) return srs_item_rows(up_rows, dn_rows);
+  const int r = dn_rows < kSrsLongRow ? kItemElems / std::max(1, dn_rows)
+                                      : std::min(kTileRows, std::max(4, std::min(24576, srs_item_elems()) / dn_rows & ~3));
   return std::max(1, std::min(r, up_rows));
 }
 

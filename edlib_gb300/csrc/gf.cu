@@ -153,8 +153,8 @@ void run_lanczos_ff(edgpu_model *m, std::vector<LzJob<double> *> &jobs, int nlan
     launch_convert<ffloat>(J.buf[0].as<double>(), J.buf[0].as<ffloat>(), s.dim, c->stream);
     J.alpha = DBuf(c->alloc, sizeof(double) * nlanc);
     J.beta = DBuf(c->alloc, sizeof(double) * (nlanc + 1));
-    J.part_a = DBuf(c->alloc, sizeof(double) * s.nitems);
-    J.part_b = DBuf(c->alloc, sizeof(double) * s.nitems);
+    J.part_a = DBuf(c->alloc, sizeof(double) * s.lz_nitems);
+    J.part_b = DBuf(c->alloc, sizeof(double) * s.lz_nitems);
     J.scal = DBuf(c->alloc, sizeof(double) * 2);
     J.state = DBuf(c->alloc, sizeof(int) * 4);
     CK(cudaMemsetAsync(J.alpha.p, 0, sizeof(double) * nlanc, c->stream));
@@ -163,9 +163,9 @@ void run_lanczos_ff(edgpu_model *m, std::vector<LzJob<double> *> &jobs, int nlan
     CK(cudaMemsetAsync(J.state.p, 0, sizeof(int) * 4, c->stream));
     LzTask<ffloat> &t = tasks[q];
     t.op = s.dop<ffloat>();
-    t.srs_rows = s.srs_rows;
+    t.srs_rows = s.lz_rows;
     t.item_begin = (int)item_task.size();
-    t.nitems = s.nitems;
+    t.nitems = s.lz_nitems;
     for (int b = 0; b < 3; ++b) t.buf[b] = J.buf[b].as<ffloat>();
     t.alpha = J.alpha.as<double>();
     t.beta = J.beta.as<double>();
@@ -174,8 +174,8 @@ void run_lanczos_ff(edgpu_model *m, std::vector<LzJob<double> *> &jobs, int nlan
     t.scal = J.scal.as<double>();
     t.state = J.state.as<int>();
     t.nlanc_max = nlanc;
-    for (int it = 0; it < s.nitems; ++it) item_task.push_back((int)q);
-    merge_shape(shape, mv_shape<double>(s));  // float-float elements take the room of FP64 ones
+    for (int it = 0; it < s.lz_nitems; ++it) item_task.push_back((int)q);
+    merge_shape(shape, mv_shape<double>(s, true));  // float-float elements take the room of FP64 ones
   }
   DBuf dt = upload(c, tasks), dm = upload(c, item_task);
   for (int it = 0; it < nlanc; ++it)
@@ -211,8 +211,8 @@ void run_lanczos(edgpu_model *m, std::vector<LzJob<T> *> &jobs, int nlanc, bool 
     Sector &s = *J.s;
     J.alpha = DBuf(c->alloc, sizeof(double) * nlanc);
     J.beta = DBuf(c->alloc, sizeof(double) * (nlanc + 1));
-    J.part_a = DBuf(c->alloc, sizeof(double) * s.nitems);
-    J.part_b = DBuf(c->alloc, sizeof(double) * s.nitems);
+    J.part_a = DBuf(c->alloc, sizeof(double) * s.lz_nitems);
+    J.part_b = DBuf(c->alloc, sizeof(double) * s.lz_nitems);
     J.scal = DBuf(c->alloc, sizeof(double) * 2);
     J.state = DBuf(c->alloc, sizeof(int) * 4);
     CK(cudaMemsetAsync(J.alpha.p, 0, sizeof(double) * nlanc, c->stream));
@@ -221,9 +221,9 @@ void run_lanczos(edgpu_model *m, std::vector<LzJob<T> *> &jobs, int nlanc, bool 
     CK(cudaMemsetAsync(J.state.p, 0, sizeof(int) * 4, c->stream));
     LzTask<T> &t = tasks[q];
     t.op = s.dop<T>();
-    t.srs_rows = s.srs_rows;
+    t.srs_rows = s.lz_rows;
     t.item_begin = (int)item_task.size();
-    t.nitems = s.nitems;
+    t.nitems = s.lz_nitems;
     for (int b = 0; b < 3; ++b) t.buf[b] = J.buf[b].template as<T>();
     t.alpha = J.alpha.template as<double>();
     t.beta = J.beta.template as<double>();
@@ -232,8 +232,8 @@ void run_lanczos(edgpu_model *m, std::vector<LzJob<T> *> &jobs, int nlanc, bool 
     t.scal = J.scal.template as<double>();
     t.state = J.state.template as<int>();
     t.nlanc_max = nlanc;
-    for (int it = 0; it < s.nitems; ++it) item_task.push_back((int)q);
-    merge_shape(shape, mv_shape<T>(s));
+    for (int it = 0; it < s.lz_nitems; ++it) item_task.push_back((int)q);
+    merge_shape(shape, mv_shape<T>(s, true));
   }
   DBuf dt = upload(c, tasks), dm = upload(c, item_task);
   for (int it = 0; it < nlanc; ++it)

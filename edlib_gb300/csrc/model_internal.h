@@ -103,8 +103,8 @@ struct SpinCsr {
   DBuf len, ell_col, ell_v64, ell_v32;  // k-major copy (SectorOp::dn_ell_*)
   DBuf uh64, uh32, uhff;           // the CSR entries as (column, value) pairs
   DBuf slot1, lv64, lv32, lvff;    // k-major entries in the order of a two-pass sector (SectorOp::long_*)
-  DBuf tlen1, tlen2, tlen4;
-  DBuf slot4, slot2, sv64, sv32, svff;  // k-major entries in the tiles' order (SectorOp::dn_slot, dn_sval)
+  DBuf tlen1;
+  DBuf slot4, slot2;               // tile slots of the k-major columns, four and two columns per lane (SectorOp::dn_slot)
   DBuf vff, ell_vff;                     // float-float values (built on first use, ensure_ff)
   std::vector<int> hrp;            // host copy of the row pointers
   DBuf vu_cnt, vu_ent;             // up spin: entries of the product interaction terms (SectorOp::vu_*)
@@ -124,9 +124,10 @@ struct Sector {
   DBuf diagff;             // float-float tables of an SRS sector, built on first use (ensure_ff)
   SectorOp<ffloat> opff{};
   DBuf dopff;
-  int srs_rows = 1, nitems = 1;
+  int srs_rows = 1, nitems = 1;        // items of products and eigen-solver steps
+  int lz_rows = 1, lz_nitems = 1;      // items of recurrences (lz_item_rows)
+  int up_kmax = 0;                     // SRS: up hops of the longest row
   bool complete = false;  // the tables are known to be built (edgpu_spmv runs on streams of its callers)
-  int up_hops_item = 0;  // most up-spin hops of one tiled item
   template <typename T> const SectorOp<T> &op() const;
   template <typename T> const SectorOp<T> *dop() const;
 };
@@ -221,7 +222,7 @@ void finish_model(edgpu_model *m);
 Sector *get_sector(edgpu_model *m, int storage, int nup, int ndn);
 // Builds (once) the float-float tables and SectorOp of a spin-resolved sector from its FP64 ones.
 void ensure_ff(edgpu_model *m, Sector *s);
-template <typename T> MvShape mv_shape(const Sector &s);
+template <typename T> MvShape mv_shape(const Sector &s, bool lz = false);
 void merge_shape(MvShape &a, const MvShape &b);
 template <typename T> void apply_h(edgpu_model *m, Sector *s, const T *x, T *y, const T *z, double cz);
 int diag_dispatch(edgpu_model *m, const edgpu_diag_params *p, int *npairs);

@@ -29,6 +29,15 @@ static_assert(kSrsLongRow >= 128, "a tile's 128 columns lie inside a row");
 
 __host__ __device__ inline size_t align16(size_t b) { return (b + 15) & ~size_t(15); }
 
+// a b, rounded by itself, and a b + c with one rounding (float-float: its own product and sum): written out where the
+// compiler could contract either of two products with their sum, so that a value does not depend on which it takes.
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ ffloat mul_rn(ffloat a, ffloat b) { return a * b; }
+__device__ __forceinline__ float madd(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double madd(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ ffloat madd(ffloat a, ffloat b, ffloat c) { return c += a * b; }
+
 template <typename T>
 __device__ __forceinline__ T transitions_term(const SectorOp<T> &op, state_t s, const Transition *L, const T *vals, int nL,
                                               const T *__restrict__ x, T acc) {
@@ -182,8 +191,8 @@ __device__ __forceinline__ void fetch_item(SrsItem<T> &d, const SectorOp<T> *opp
   d.z = z ? z + lo : nullptr;
   d.y = y + lo;
   d.slot = op.dn_slot;
-  d.ev = op.dn_sval;
-  d.len = Nd >= kSrsLongRow && Nd < kSrsVeryLong ? op.dn_tlen : op.dn_len;
+  d.ev = op.dn_ell_val;
+  d.len = op.dn_len;
   d.urp = op.up_rp + u0;
   d.uh = op.up_hop;
   d.dot = lz ? lz->part_a + li : nullptr;
@@ -254,17 +263,17 @@ template <typename T>
 __device__ __forceinline__ Lanes<T> ldg16(const T *p) {
   return load_lanes(p, true, Lanes<T>::C);
 }
-// A lane's C elements of a row: 16 consecutive bytes (VEC), or elements 32 apart; RO: through the read-only path
+// A lane's C elements of a row: 16 consecutive bytes (VEC), or elements o apart from p; RO: through the read-only path
 // (z may be the vector being written).
 template <typename T, int C, bool VEC, bool RO = true>
-__device__ __forceinline__ void ld_tile(const T *p, T (&v)[C]) {
+__device__ __forceinline__ void ld_tile(const T *p, const int (&o)[C], T (&v)[C]) {
   if constexpr (VEC) {
     const Lanes<T> q = RO ? ldg16(p) : load16(p);
 #pragma unroll
     for (int cc = 0; cc < C; ++cc) v[cc] = q.v[cc];
   } else {
 #pragma unroll
-    for (int cc = 0; cc < C; ++cc) v[cc] = RO ? ldg_t(p + 32 * cc) : p[32 * cc];
+    for (int cc = 0; cc < C; ++cc) v[cc] = RO ? ldg_t(p + o[cc]) : p[o[cc]];
   }
 }
 
@@ -323,7 +332,7 @@ __device__ __forceinline__ void stage_interleaved(T *xs, const T *__restrict__ x
 
 // The C slots and values of one k-major entry row for a lane's columns (16-byte pieces when VEC).
 template <typename T, int C, bool VEC>
-__device__ __forceinline__ void ld_entry(const unsigned short *slot, const T *val, int (&c)[C], T (&v)[C]) {
+__device__ __forceinline__ void ld_entry(const unsigned short *slot, const T *val, const int (&o)[C], int (&c)[C], T (&v)[C]) {
   if constexpr (VEC && C == 4) {
     const uint2 q = __ldg(reinterpret_cast<const uint2 *>(slot));
     c[0] = q.x & 0xffff, c[1] = q.x >> 16, c[2] = q.y & 0xffff, c[3] = q.y >> 16;
@@ -332,9 +341,9 @@ __device__ __forceinline__ void ld_entry(const unsigned short *slot, const T *va
     c[0] = q & 0xffff, c[1] = q >> 16;
   } else {
 #pragma unroll
-    for (int cc = 0; cc < C; ++cc) c[cc] = __ldg(slot + 32 * cc);
+    for (int cc = 0; cc < C; ++cc) c[cc] = __ldg(slot + o[cc]);
   }
-  ld_tile<T, C, VEC>(val, v);
+  ld_tile<T, C, VEC>(val, o, v);
 }
 
 // The up hops of an item in shared memory: row r's at [rp[r], rp[r + 1]), c = the source row's offset in x;
@@ -346,72 +355,89 @@ struct ItemHops {
 };
 
 // A thread's part of a tile of the SRS sweep: rows rg .. rg + 3 of the item (those below nrows), columns from c0 on
-// (kVec: C consecutive ones; else 32 apart, those below cb not its own).  Lanes that are not `mine`, columns below cb
-// and rows past the item's end repeat others' and store nothing: every load is in bounds without a predicate.
+// (kVec: C consecutive ones; else 32 apart).  Columns below cb are another tile's, columns past the row's end (MD) and the
+// lanes that are not `mine` repeat others, and so do rows past the item's end; all of them store nothing: every load is
+// in bounds without a predicate.
 // What bounds it: L1 and shared-memory wavefronts, then issue slots.  Rows apart in shared memory (each down-hop
 // entry 16 address computations and 16 scalar loads per thread) took 110 thread instructions per state.  Here an
 // entry is one 16-byte shared-memory load per column for RI rows, and the item's up hops come from shared memory, HB
 // of them in flight per row.  Rows of 924 or 792 states start off 128-byte lines, where a warp's 4-byte accesses
 // touch two lines each: those take 16-byte accesses (the 64-vector product of the 12-orbital sector (6,6): 428 us with
-// 4-byte ones).  A column's down hops are in an order in which the eight lanes
-// of a shared-memory phase meet few bank conflicts (k_tile_schedule).  64 FP32 vectors of sector (6,6), rows of 924
-// states: 355 -> 279 us; (6,4), rows of 495: 317 -> 210 us; 14-site rows of 3432: 11.6 -> 8.3 ps per state.
-// Per element the sum runs diagonal, (c z), down hops, up hops in the reference's order, interaction.
+// 4-byte ones).
+// Per element the sum runs diagonal, (c z), down hops and up hops each in the reference's order, interaction: another
+// order (down hops dealt out so that a phase's eight lanes meet few bank conflicts) is faster, but the eigen-solver's
+// and the recurrences' vectors are then others in the last bit, which unconverged quantities magnify.
 template <typename T, int M, int HB, bool MZ, bool MD>
 __device__ __forceinline__ void srs_tile(const SrsItem<T> &it, const ItemHops<T> &hops, int rg, int cb, int c0, bool mine,
                                          const T *__restrict__ xs, DotAcc &acc) {
   using TG = TileGeom<T>;
   constexpr bool VEC = M == kVec;
-  constexpr int R = TG::R, C = TG::C, RI = TG::RI, NP = TG::NP, S = VEC ? 1 : 32;
+  constexpr int R = TG::R, C = TG::C, RI = TG::RI, NP = TG::NP;
   const int Nd = it.Nd;
   const Lanes<T> *__restrict__ xv = reinterpret_cast<const Lanes<T> *>(xs) + (rg / RI) * Nd;
-  auto slot = [&](int cc) { return VEC ? c0 / C + cc * (Nd / C) : M == kOdd ? c0 + S * cc : tile_slot(c0 + S * cc, Nd, C); };
+  int o[C];  // the columns, from c0
+#pragma unroll
+  for (int cc = 0; cc < C; ++cc) o[cc] = VEC ? cc : MD ? min(32 * cc, Nd - 1 - c0) : 32 * cc;
+  auto own = [&](int cc) { return VEC ? mine : MD ? c0 + 32 * cc < Nd : c0 + 32 * cc >= cb; };
+  auto slot = [&](int cc) { return VEC ? c0 / C + cc * (Nd / C) : M == kOdd ? c0 + o[cc] : tile_slot(c0 + o[cc], Nd, C); };
   auto row = [&](int r) { return min(rg + r, it.nrows - 1) * Nd + c0; };
   T a[R][C];
 #pragma unroll
-  for (int r = 0; r < R; ++r) ld_tile<T, C, VEC>(it.dg + row(r), a[r]);
-#pragma unroll
-  for (int p = 0; p < NP; ++p)
-#pragma unroll
-    for (int cc = 0; cc < C; ++cc) {
-      const Lanes<T> q = xv[p * Nd + slot(cc)];
-#pragma unroll
-      for (int i = 0; i < RI; ++i) a[p * RI + i][cc] = a[p * RI + i][cc] * q.v[i];
-    }
+  for (int r = 0; r < R; ++r) ld_tile<T, C, VEC>(it.dg + row(r), o, a[r]);
   if (MZ && it.z) {
+    // a + c z; whole groups of four rows and rows of no whole 16-byte pieces round c z first, others the diagonal's term
+    const bool first = !VEC || rg + R <= it.nrows;
+    T zq[R][C];
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      T zq[C];
-      ld_tile<T, C, VEC, false>(it.z + row(r), zq);
+    for (int r = 0; r < R; ++r) ld_tile<T, C, VEC, false>(it.z + row(r), o, zq[r]);
 #pragma unroll
-      for (int cc = 0; cc < C; ++cc) a[r][cc] = a[r][cc] + it.c * zq[cc];
-    }
+    for (int p = 0; p < NP; ++p)
+#pragma unroll
+      for (int cc = 0; cc < C; ++cc) {
+        const Lanes<T> q = xv[p * Nd + slot(cc)];
+#pragma unroll
+        for (int i = 0; i < RI; ++i) {
+          T &e = a[p * RI + i][cc];
+          const T z = zq[p * RI + i][cc];
+          if constexpr (std::is_same<T, ffloat>::value) e = e * q.v[i] + it.c * z;
+          else e = first ? madd(e, q.v[i], mul_rn(it.c, z)) : madd(it.c, z, mul_rn(e, q.v[i]));
+        }
+      }
+  } else {
+#pragma unroll
+    for (int p = 0; p < NP; ++p)
+#pragma unroll
+      for (int cc = 0; cc < C; ++cc) {
+        const Lanes<T> q = xv[p * Nd + slot(cc)];
+#pragma unroll
+        for (int i = 0; i < RI; ++i) a[p * RI + i][cc] = mul_rn(a[p * RI + i][cc], q.v[i]);
+      }
   }
   {
     int kk = 0;
 #pragma unroll
-    for (int cc = 0; cc < C; ++cc) kk = max(kk, ldg_t(it.len + c0 + S * cc));
+    for (int cc = 0; cc < C; ++cc) kk = max(kk, ldg_t(it.len + c0 + o[cc]));
     if (!mine) kk = 0;  // lanes past the row's end sum nothing
     const unsigned short *__restrict__ es = it.slot + c0;
     const T *__restrict__ ev = it.ev + c0;
     const int ld = it.ld;
     int hc[C];
     T hv[C];
-    if (kk > 0) ld_entry<T, C, VEC>(es, ev, hc, hv);
+    if (kk > 0) ld_entry<T, C, VEC>(es, ev, o, hc, hv);
 #pragma unroll 1
     for (int k = 0; k < kk; ++k) {
       int nc[C];
       T nv[C];
       es += ld;
       ev += ld;
-      if (k + 1 < kk) ld_entry<T, C, VEC>(es, ev, nc, nv);
+      if (k + 1 < kk) ld_entry<T, C, VEC>(es, ev, o, nc, nv);
 #pragma unroll
       for (int cc = 0; cc < C; ++cc)
 #pragma unroll
         for (int p = 0; p < NP; ++p) {
           const Lanes<T> q = xv[p * Nd + hc[cc]];
 #pragma unroll
-          for (int i = 0; i < RI; ++i) a[p * RI + i][cc] += hv[cc] * q.v[i];
+          for (int i = 0; i < RI; ++i) a[p * RI + i][cc] = madd(hv[cc], q.v[i], a[p * RI + i][cc]);
         }
 #pragma unroll
       for (int cc = 0; cc < C; ++cc) hc[cc] = nc[cc], hv[cc] = nv[cc];
@@ -438,7 +464,7 @@ __device__ __forceinline__ void srs_tile(const SrsItem<T> &it, const ItemHops<T>
         for (int q = 0; q < HB; ++q) {
           const Hop<T> hp = hops.hop[h + q < n[r] ? k0[r] + h + q : none];
           v[r][q] = hp.v;
-          ld_tile<T, C, VEC>(xc + hp.c, xq[r][q]);
+          ld_tile<T, C, VEC>(xc + hp.c, o, xq[r][q]);
         }
 #pragma unroll
       for (int r = 0; r < R; ++r)
@@ -446,7 +472,7 @@ __device__ __forceinline__ void srs_tile(const SrsItem<T> &it, const ItemHops<T>
         for (int q = 0; q < HB; ++q)
           if (h + q < n[r]) {  // uniform over the warp
 #pragma unroll
-            for (int cc = 0; cc < C; ++cc) a[r][cc] += v[r][q] * xq[r][q][cc];
+            for (int cc = 0; cc < C; ++cc) a[r][cc] = madd(v[r][q], xq[r][q][cc], a[r][cc]);
           }
     }
   }
@@ -457,7 +483,7 @@ __device__ __forceinline__ void srs_tile(const SrsItem<T> &it, const ItemHops<T>
       RowPart<T, C> p;
 #pragma unroll
       for (int cc = 0; cc < C; ++cc) p.v[cc] = a[r][cc];
-      p = srs_vloc<T, C, S>(it.op, it.u0 + rg + r, c0, it.x, p);
+      p = srs_vloc<T, C, VEC ? 1 : 32>(it.op, it.u0 + rg + r, c0, it.x, p);
 #pragma unroll
       for (int cc = 0; cc < C; ++cc) a[r][cc] = p.v[cc];
     }
@@ -467,22 +493,23 @@ __device__ __forceinline__ void srs_tile(const SrsItem<T> &it, const ItemHops<T>
     } else {
 #pragma unroll
       for (int cc = 0; cc < C; ++cc)
-        if (c0 + S * cc >= cb) y[S * cc] = renorm(a[r][cc]);
+        if (own(cc)) y[o[cc]] = renorm(a[r][cc]);
     }
     if (MD && it.dot) {
 #pragma unroll
       for (int cc = 0; cc < C; ++cc)
-        if (VEC ? mine : c0 + S * cc >= cb) dot_add(acc, xv[(r / RI) * Nd + slot(cc)].v[r % RI], a[r][cc]);
+        if (own(cc)) dot_add(acc, xv[(r / RI) * Nd + slot(cc)].v[r % RI], a[r][cc]);
     }
   }
 }
 
 // The tiles of a staged item; the thread's part of <x, y>.  Either a warp per tile of 4 rows x W columns, so that a
-// shared-memory phase's eight lanes hold the columns k_tile_schedule put together; past the row's end kVec lanes take
+// shared-memory phase's eight lanes hold neighbouring columns; past the row's end kVec lanes take
 // the last columns again (the same addresses as their owner's, no extra wavefront), the others' tiles move back to
 // end with the row.  Or the units of a kVec item numbered through, a thread each, rows ending inside a warp: for
 // 8-byte types, bound by arithmetic, whose cost does not fall with idle lanes, and for rows that leave more than a
-// ninth of the tiles' columns empty (FP32 rows of 220 states).
+// ninth of the tiles' columns empty (FP32 rows of 220 states).  With dot products (MD) a thread's elements are part of
+// the sums' values: kVec units numbered through, other tiles not moved.
 template <typename T, int M, int HB, bool MZ, bool MD>
 __device__ __forceinline__ DotAcc srs_tiles(const SrsItem<T> &it, const ItemHops<T> &hops, const T *__restrict__ xs) {
   using TG = TileGeom<T>;
@@ -490,13 +517,13 @@ __device__ __forceinline__ DotAcc srs_tiles(const SrsItem<T> &it, const ItemHops
   DotAcc acc;
   dot_init(acc);
   const int ngr = (it.nrows + TG::R - 1) / TG::R, ncb = (it.Nd + TG::W - 1) / TG::W, lane = threadIdx.x & 31;
-  const bool linear = M == kVec && (sizeof(T) == 8 || 8 * ncb * TG::W > 9 * it.Nd);
+  const bool linear = M == kVec && (sizeof(T) == 8 || MD || 8 * ncb * TG::W > 9 * it.Nd);
   const int per = linear ? it.Nd / C : ncb;
 #pragma unroll 1
   for (int unit = linear ? threadIdx.x : threadIdx.x >> 5; unit < ngr * per; unit += linear ? kMvBlock : kMvBlock / 32) {
     const int g = unit / per, q = unit - g * per;
-    const int cb = linear ? 0 : q * TG::W, want = linear ? q * C : M == kVec ? cb + C * lane : min(cb, it.Nd - TG::W) + lane;
-    srs_tile<T, M, HB, MZ, MD>(it, hops, g * TG::R, cb, M == kVec ? min(want, it.Nd - C) : want, M != kVec || want < it.Nd,
+    const int cb = linear ? 0 : q * TG::W, want = linear ? q * C : M == kVec ? cb + C * lane : (MD ? cb : min(cb, it.Nd - TG::W)) + lane;
+    srs_tile<T, M, HB, MZ, MD>(it, hops, g * TG::R, cb, M == kVec ? min(want, it.Nd - C) : want, want < it.Nd,
                                xs, acc);
   }
   return acc;
@@ -633,16 +660,14 @@ __device__ __noinline__ DotAcc srs_longrow(const SrsItem<T> &it, const T *__rest
 // down-hop entry, loaded once, serves RI rows.  Per element the sums of the tiles, in the reference's order.
 // 12-orbital impurity, rows of 66 states, FP32: 21 ps per state, rows of 12: 25 (20 and 24 one element per
 // thread, the CSR entry by entry; 33 and 53 that way in a block of two per SM).
-template <typename T, bool MZ, bool MD>
-__device__ __noinline__ DotAcc srs_short(const SrsItem<T> &it, const ItemHops<T> &hops, bool near, const T *__restrict__ xs) {
+template <typename T, bool MZ>
+__device__ __noinline__ void srs_short(const SrsItem<T> &it, const ItemHops<T> &hops, bool near, const T *__restrict__ xs) {
   constexpr int RI = Lanes<T>::C;
   const SectorOp<T> &op = *it.op;
   const Lanes<T> *__restrict__ xv = reinterpret_cast<const Lanes<T> *>(xs);
   const int Nd = it.Nd, ld = it.ld, n = (it.nrows + RI - 1) / RI * Nd;
   const int *__restrict__ ecol = op.dn_ell_col;
   const T *__restrict__ eval = op.dn_ell_val;
-  DotAcc acc;
-  dot_init(acc);
   int g = threadIdx.x / Nd, d = threadIdx.x - g * Nd;
   const int gs = kMvBlock / Nd, ds = kMvBlock - gs * Nd;
   for (int e = threadIdx.x; e < n; e += kMvBlock) {
@@ -654,10 +679,10 @@ __device__ __noinline__ DotAcc srs_short(const SrsItem<T> &it, const ItemHops<T>
     for (int r = 0; r < RI; ++r) ro[r] = (g * RI + min(r, nr - 1)) * Nd + d;
     T a[RI];
 #pragma unroll
-    for (int r = 0; r < RI; ++r) a[r] = ldg_t(it.dg + ro[r]) * own.v[r];
+    for (int r = 0; r < RI; ++r) a[r] = mul_rn(ldg_t(it.dg + ro[r]), own.v[r]);
     if (MZ && it.z) {
 #pragma unroll
-      for (int r = 0; r < RI; ++r) a[r] = a[r] + it.c * it.z[ro[r]];
+      for (int r = 0; r < RI; ++r) a[r] = madd(it.c, it.z[ro[r]], a[r]);
     }
     const int kk = ldg_t(it.len + d);
 #pragma unroll 4
@@ -665,7 +690,7 @@ __device__ __noinline__ DotAcc srs_short(const SrsItem<T> &it, const ItemHops<T>
       const Lanes<T> q = xg[ldg_t(ecol + k * ld + d)];
       const T v = ldg_t(eval + k * ld + d);
 #pragma unroll
-      for (int r = 0; r < RI; ++r) a[r] += v * q.v[r];
+      for (int r = 0; r < RI; ++r) a[r] = madd(v, q.v[r], a[r]);
     }
     int k0[RI], nh[RI], nmax = 0;
 #pragma unroll
@@ -701,7 +726,7 @@ __device__ __noinline__ DotAcc srs_short(const SrsItem<T> &it, const ItemHops<T>
       for (int q = 0; q < 4; ++q)
 #pragma unroll
         for (int r = 0; r < RI; ++r)
-          if (h + q < nh[r]) a[r] += v[q][r] * xq[q][r];
+          if (h + q < nh[r]) a[r] = madd(v[q][r], xq[q][r], a[r]);
     }
     if (it.vloc) {
       RowPart<T, RI> p;
@@ -715,11 +740,53 @@ __device__ __noinline__ DotAcc srs_short(const SrsItem<T> &it, const ItemHops<T>
     for (int r = 0; r < RI; ++r) {
       if (r >= nr) continue;
       it.y[ro[r]] = renorm(a[r]);
-      if (MD && it.dot) dot_add(acc, own.v[r], a[r]);
     }
     g += gs;
     d += ds;
     if (d >= Nd) d -= Nd, ++g;
+  }
+}
+
+// The same with dot products: a thread takes one element at a time, e = threadIdx.x, + kMvBlock, ... over the item, which
+// is part of the value of <x, y>.
+template <typename T, bool MZ>
+__device__ __noinline__ DotAcc srs_flat(const SrsItem<T> &it, const ItemHops<T> &hops, bool near, const T *__restrict__ xs) {
+  constexpr int RI = Lanes<T>::C;
+  const SectorOp<T> &op = *it.op;
+  const int Nd = it.Nd, ld = it.ld, n = it.nrows * Nd, first = ldg_t(it.urp);
+  const int *__restrict__ ecol = op.dn_ell_col;
+  const T *__restrict__ eval = op.dn_ell_val;
+  DotAcc acc;
+  dot_init(acc);
+  int r = threadIdx.x / Nd, d = threadIdx.x - r * Nd;
+  const int rs = kMvBlock / Nd, ds = kMvBlock - rs * Nd;
+  for (int e = threadIdx.x; e < n; e += kMvBlock) {
+    const T *__restrict__ xg = xs + (r / RI) * Nd * RI + r % RI;
+    const T xv = xg[d * RI];
+    T a = mul_rn(ldg_t(it.dg + e), xv);
+    if (MZ && it.z) a = madd(it.c, it.z[e], a);
+    const int kk = ldg_t(it.len + d);
+#pragma unroll 4
+    for (int k = 0; k < kk; ++k) a = madd(ldg_t(eval + k * ld + d), xg[ldg_t(ecol + k * ld + d) * RI], a);
+    const int k0 = ldg_t(it.urp + r), nh = ldg_t(it.urp + r + 1) - k0;
+    const T *__restrict__ xd = it.x + d;
+#pragma unroll 4
+    for (int h = 0; h < nh; ++h) {
+      Hop<T> hp;
+      if (near) {
+        hp = hops.hop[k0 - first + h];
+      } else {
+        hp = ldg_hop(it.uh + k0 + h);
+        hp.c *= Nd;
+      }
+      a = madd(hp.v, ldg_t(xd + hp.c), a);
+    }
+    if (it.vloc) a = srs_vloc<T, 1, 1>(it.op, it.u0 + r, d, it.x, RowPart<T, 1>{{a}}).v[0];
+    it.y[e] = renorm(a);
+    dot_add(acc, xv, a);
+    r += rs;
+    d += ds;
+    if (d >= Nd) d -= Nd, ++r;
   }
   return acc;
 }
@@ -929,13 +996,14 @@ __global__ void __launch_bounds__(kMvBlock, MB) k_srs_mv(Src src, int nitems, in
     if (threadIdx.x == kMvBlock - 32) fetch(i + gridDim.x, items[p ^ 1]);  // the next item's description
     if (!tile && !small) cp_async_wait_all();
     __syncthreads();
-    DotAcc acc;
+    DotAcc acc{};
     if (tile) {
       if (vec) acc = srs_tiles<T, kVec, HB, MZ, MD>(it, hops, xs);
       else if (!whole) acc = srs_tiles<T, kOdd, HB, MZ, MD>(it, hops, xs);
       else acc = srs_tiles_off<T, MZ, MD>(it, hops, xs);
     } else if (small) {
-      acc = srs_short<T, MZ, MD>(it, hops, near, xs);
+      if constexpr (MD) acc = srs_flat<T, MZ>(it, hops, near, xs);
+      else srs_short<T, MZ>(it, hops, near, xs);
     } else {
       acc = srs_longrow<T, MZ, MD>(it, nel <= xs_cap ? xs : it.xi);
     }

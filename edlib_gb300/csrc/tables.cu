@@ -287,34 +287,40 @@ template void launch_pack_hops<float>(const int *, const float *, long long, Hop
 template void launch_pack_hops<double>(const int *, const double *, long long, Hop<double> *, cudaStream_t);
 template void launch_pack_hops<ffloat>(const int *, const ffloat *, long long, Hop<ffloat> *, cudaStream_t);
 
-// The order of a column's down hops in a tile.  A 16-byte shared-memory load of a warp runs in four phases of eight
-// lanes; lanes whose slots agree modulo 8 (but differ) take one wavefront more each.  The eight lanes of a phase may
-// take their entries in any order, so per group of eight columns (C apart in rows of a multiple of C states, else
-// side by side: spmv.cuh, srs_tile) entries are dealt in rounds: lanes with most entries left first, each the entry
-// whose bank is least used in this round, among those the bank with most entries left; a lane that would meet a conflict
-// and has rounds to spare waits, reading what the round's first lane reads (value 0).  On 924-state rows of the
-// 12-orbital impurity 2.28 -> 1.79 wavefronts per load, 495-state rows 1.90 -> 1.08 (counted from the hop pattern).
-__global__ void k_tile_schedule(const int *ell_col, const int *len, int rows, int ld, int kmax, int C, unsigned short *slot,
+__global__ void k_tile_slots(const int *ell_col, int n, int rows, int C, unsigned short *slot) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    slot[i] = (unsigned short)tile_slot(ell_col[i], rows, C);
+}
+void launch_tile_slots(const int *ell_col, int n, int rows, int C, unsigned short *slot, cudaStream_t st) {
+  k_tile_slots<<<std::max(1, std::min(1024, (n + 255) / 256)), 256, 0, st>>>(ell_col, n, rows, C, slot); note_launch();
+}
+
+// The order of a row's hops in the two-pass kernels, one row per lane.  A 16-byte shared-memory load of a warp runs in
+// four phases of eight lanes; lanes whose places agree modulo 8 (but differ) take one wavefront more each.  The eight
+// lanes of a phase may take their entries in any order, so per group of eight rows entries are dealt in rounds: lanes with
+// most entries left first, each the entry whose bank is least used in this round, among those the bank with most entries
+// left; a lane that would meet a conflict and has rounds to spare waits, reading what the round's first lane reads (value
+// 0).  (The tiles keep the matrix' order: eigen-solves and recurrences add in it, and sums in another order are other
+// values.  There a load takes 1.8 to 2.5 wavefronts; dealt out it took 1.1 to 1.8.)
+__global__ void k_long_schedule(const int *ell_col, const int *len, int rows, int ld, int kmax, unsigned short *slot,
                                 short *order, int *tlen) {
-  // the group's slots at hand: lane q's entry e at at[(e * 8 + q) * 32], for rows of at most 64 entries
+  // the group's columns at hand: lane q's entry e at at[(e * 8 + q) * 32], for rows of at most 64 entries
   extern __shared__ unsigned short schedule_smem[];
   unsigned short *at = schedule_smem + threadIdx.x;
-  const int W = 32 * C, ngroups = (rows + W - 1) / W * C * 4;
+  const int ngroups = (rows + 7) / 8;
   for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < ngroups; g += gridDim.x * blockDim.x) {
-    const int tile = g / (4 * C), cc = g / 4 % C, ph = g % 4;
     int col[8], left[8], cnt[8];
     unsigned long long rem[8];
     int nmax = 0;
     for (int b = 0; b < 8; ++b) cnt[b] = 0;
     for (int q = 0; q < 8; ++q) {
-      const int lane = 8 * ph + q;
-      const int d = tile * W + (rows % C ? 32 * cc + lane : C * lane + cc);
+      const int d = 8 * g + q;
       col[q] = d < rows ? d : -1;
       left[q] = d < rows ? len[d] : 0;
       rem[q] = left[q] >= 64 ? ~0ull : (1ull << left[q]) - 1;
       nmax = max(nmax, left[q]);
       for (int e = 0; e < left[q]; ++e) {
-        const int s = tile_slot(ell_col[e * ld + d], rows, C);
+        const int s = ell_col[e * ld + d];
         if (e < 64) at[(e * 8 + q) * 32] = (unsigned short)s;
         ++cnt[s & 7];
       }
@@ -338,7 +344,7 @@ __global__ void k_tile_schedule(const int *ell_col, const int *len, int rows, in
           if (best < 0 || used[b] < bu || (used[b] == bu && cnt[b] > bc)) best = e, bu = used[b], bc = cnt[b];
         }
         if (nmax <= 64 && bu > 0 && left[q] < nmax - k) continue;
-        const int s = best < 64 ? at[(best * 8 + q) * 32] : tile_slot(ell_col[best * ld + col[q]], rows, C);
+        const int s = best < 64 ? at[(best * 8 + q) * 32] : ell_col[best * ld + col[q]];
         ++used[s & 7];
         --cnt[s & 7];
         --left[q];
@@ -350,16 +356,16 @@ __global__ void k_tile_schedule(const int *ell_col, const int *len, int rows, in
         if (col[q] < 0) continue;
         const int o = k * ld + col[q];
         order[o] = (short)pick[q];
-        slot[o] = (unsigned short)(pick[q] < 0 ? (first >= 0 ? first : tile_slot(col[q], rows, C))
-                                   : pick[q] < 64 ? at[(pick[q] * 8 + q) * 32] : tile_slot(ell_col[pick[q] * ld + col[q]], rows, C));
+        slot[o] = (unsigned short)(pick[q] < 0 ? (first >= 0 ? first : col[q])
+                                   : pick[q] < 64 ? at[(pick[q] * 8 + q) * 32] : ell_col[pick[q] * ld + col[q]]);
       }
     }
   }
 }
-void launch_tile_schedule(const int *ell_col, const int *len, int rows, int ld, int kmax, int C, unsigned short *slot,
-                          short *order, int *tlen, cudaStream_t st) {
-  const int ngroups = (rows + 32 * C - 1) / (32 * C) * C * 4;
-  k_tile_schedule<<<(ngroups + 31) / 32, 32, sizeof(unsigned short) * 32 * 8 * std::min(kmax, 64), st>>>(ell_col, len, rows, ld, kmax, C, slot, order, tlen); note_launch();
+void launch_long_schedule(const int *ell_col, const int *len, int rows, int ld, int kmax, unsigned short *slot, short *order,
+                          int *tlen, cudaStream_t st) {
+  const int ngroups = (rows + 7) / 8;
+  k_long_schedule<<<(ngroups + 31) / 32, 32, sizeof(unsigned short) * 32 * 8 * std::min(kmax, 64), st>>>(ell_col, len, rows, ld, kmax, slot, order, tlen); note_launch();
 }
 
 template <typename T>
