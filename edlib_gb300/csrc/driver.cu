@@ -123,56 +123,44 @@ int err_flag(edgpu_ctx *c, const DBuf &e) {
 }
 
 // ============================================================================ model upload
-// The spin-resolved operator's split of the interaction terms (VProd).  The down matrices of one particle number
-// take up to nW kW C(ns, k) entries of 24 bytes: a tensor dense enough to need more than 256 MB at half filling
-// keeps the transition list.
+// The interaction terms of the spin-resolved operator as pairs of one-spin hops (VProd).  A model with a term inside one
+// spin, which has no place in the tables, keeps the transition list, so that every element sums its terms in their order;
+// so does one whose up entries would take more than 256 MB at half filling.
 static void split_interaction(edgpu_model *m) {
   edgpu_ctx *c = m->ctx;
   const int ns = m->ns;
-  VProd &P = m->vprod;
-  std::map<std::pair<int, int>, std::map<std::pair<int, int>, double>> prod;  // (I, K) -> (J, L) -> value
-  for (auto &t : m->V) {
+  VProd P;
+  std::map<std::pair<int, int>, int> down;  // (J, L) -> g
+  for (size_t q = 0; q < m->V.size(); ++q) {
+    const Transition &t = m->V[q];
     const bool dn1 = t.k >= ns, dn2 = t.l >= ns;  // spins of the k -> i and l -> j halves
     if (dn1 == dn2) {
-      if (t.k != t.l && t.i != t.j) m->Vs.push_back(t);  // equal indices annihilate every state
-    } else if (!dn1) {
-      prod[{t.i, t.k}][{t.j - ns, t.l - ns}] += t.value;
-    } else {
-      prod[{t.j, t.l}][{t.i - ns, t.k - ns}] += t.value;
+      if (t.k != t.l && t.i != t.j) return;
+      continue;  // equal indices annihilate every state
     }
-  }
-  for (auto &h : prod) {
-    P.upI.push_back(h.first.first);
-    P.upK.push_back(h.first.second);
-    P.off.push_back((int)P.dnJ.size());
-    for (auto &g : h.second) {
-      P.dnJ.push_back(g.first.first);
-      P.dnL.push_back(g.first.second);
-      P.val.push_back(g.second);
+    P.upI.push_back(dn1 ? t.j : t.i);
+    P.upK.push_back(dn1 ? t.l : t.k);
+    const std::pair<int, int> jl(dn1 ? t.i - ns : t.j - ns, dn1 ? t.k - ns : t.l - ns);
+    auto it = down.find(jl);
+    if (it == down.end()) {
+      it = down.emplace(jl, (int)P.dnJ.size()).first;
+      P.dnJ.push_back(jl.first);
+      P.dnL.push_back(jl.second);
     }
-    P.kW = std::max(P.kW, (int)h.second.size());
+    P.g.push_back(it->second);
+    P.t.push_back((int)q);
   }
-  P.off.push_back((int)P.dnJ.size());
   const size_t nW = P.upI.size();
-  if (nW * (size_t)P.kW * (size_t)binom_at_host(ns, ns / 2) * 24 > ((size_t)256 << 20)) {
-    P = VProd();
-    m->Vs = m->V;
-  } else if (nW > 0) {
-    P.dI = upload(c, P.upI);
-    P.dK = upload(c, P.upK);
-    P.doff = upload(c, P.off);
-    P.dJ = upload(c, P.dnJ);
-    P.dL = upload(c, P.dnL);
-    P.dval = upload(c, P.val);
-    P.dev = DevVProd{(int)nW, P.kW, P.dI.as<int>(), P.dK.as<int>(), P.doff.as<int>(), P.dJ.as<int>(), P.dL.as<int>(),
-                     P.dval.as<double>()};
-  }
-  std::vector<double> v64;
-  std::vector<float> v32;
-  for (auto &t : m->Vs) v64.push_back(t.value), v32.push_back((float)t.value);
-  m->dVs = upload(c, m->Vs);
-  m->dVsv64 = upload(c, v64);
-  m->dVsv32 = upload(c, v32);
+  if (nW == 0 || nW * sizeof(int4) * (size_t)binom_at_host(ns, ns / 2) > ((size_t)256 << 20)) return;
+  P.dI = upload(c, P.upI);
+  P.dK = upload(c, P.upK);
+  P.dg = upload(c, P.g);
+  P.dt = upload(c, P.t);
+  P.dJ = upload(c, P.dnJ);
+  P.dL = upload(c, P.dnL);
+  P.dev = DevVProd{(int)nW, (int)P.dnJ.size(), P.dI.as<int>(), P.dK.as<int>(), P.dg.as<int>(), P.dt.as<int>(),
+                   P.dJ.as<int>(), P.dL.as<int>()};
+  m->vprod = std::move(P);
 }
 
 void finish_model(edgpu_model *m) {
@@ -309,21 +297,13 @@ SpinCsr *get_spin(edgpu_model *m, int spin, int k) {
   const DevVProd &vp = m->vprod.dev;
   if (vp.nW > 0 && spin == 0) {
     s->vu_cnt = DBuf(c->alloc, sizeof(int) * rows);
-    s->vu_ent = DBuf(c->alloc, sizeof(int2) * (size_t)rows * vp.nW);
+    s->vu_ent = DBuf(c->alloc, sizeof(int4) * (size_t)rows * vp.nW);
     launch_vprod_up(m->dm, vp, k, (int)rows, m->dbasis.as<int>() + m->basis_off[k], s->vu_cnt.as<int>(),
-                    s->vu_ent.as<int2>(), c->stream);
+                    s->vu_ent.as<int4>(), c->stream);
   } else if (vp.nW > 0) {
-    s->vd_cells = (long long)vp.nW * vp.kW * s->ld;
-    s->vd_len = DBuf(c->alloc, sizeof(int) * (size_t)vp.nW * s->ld);
-    s->vd_col = DBuf(c->alloc, sizeof(int) * (size_t)s->vd_cells);
-    s->vd_v64 = DBuf(c->alloc, sizeof(double) * (size_t)s->vd_cells);
-    s->vd_v32 = DBuf(c->alloc, sizeof(float) * (size_t)s->vd_cells);
-    CK(cudaMemsetAsync(s->vd_len.p, 0, s->vd_len.bytes, c->stream));
-    CK(cudaMemsetAsync(s->vd_col.p, 0, s->vd_col.bytes, c->stream));
-    CK(cudaMemsetAsync(s->vd_v64.p, 0, s->vd_v64.bytes, c->stream));
-    CK(cudaMemsetAsync(s->vd_v32.p, 0, s->vd_v32.bytes, c->stream));
-    launch_vprod_dn(m->dm, vp, k, (int)rows, s->ld, m->dbasis.as<int>() + m->basis_off[k], s->vd_len.as<int>(),
-                    s->vd_col.as<int>(), s->vd_v64.as<double>(), s->vd_v32.as<float>(), c->stream);
+    s->vd_to = DBuf(c->alloc, sizeof(int) * (size_t)vp.ng * s->ld);
+    CK(cudaMemsetAsync(s->vd_to.p, 0xff, s->vd_to.bytes, c->stream));
+    launch_vprod_dn(m->dm, vp, k, (int)rows, s->ld, m->dbasis.as<int>() + m->basis_off[k], s->vd_to.as<int>(), c->stream);
   }
   SpinCsr *raw = s.get();
   m->spin[key] = std::move(s);
@@ -370,14 +350,13 @@ void fill_common(edgpu_model *m, const Sector &s, SectorOp<T> &op, const T *diag
   op.V_ = m->dV.as<Transition>();
   op.T_val = tval;
   op.V_val = vval;
-  op.nW = op.kW = 0;
+  op.nW = 0;
   op.nM = (int)(m->T.size() + m->V.size());
   op.M_ = m->dM.as<TransMask>();
   if constexpr (sizeof(T) == 4) op.M_val = m->dMv32.as<float>();
   else op.M_val = m->dMv64.as<double>();
-  op.vu_cnt = op.vd_len = op.vd_col = nullptr;
+  op.vu_cnt = op.vd_to = nullptr;
   op.vu_ent = nullptr;
-  op.vd_val = nullptr;
   for (int q = 0; q < 2; ++q) {
     op.long_slot[q] = nullptr;
     op.long_val[q] = nullptr;
@@ -396,7 +375,7 @@ void ensure_ff(edgpu_model *m, Sector *s) {
   };
   if (!m->dTvff.p) {
     conv(m->dTvff, m->dTv64, (long long)m->T.size());
-    conv(m->dVvff, m->dVsv64, (long long)m->Vs.size());
+    conv(m->dVvff, m->dVv64, (long long)m->V.size());
   }
   SpinCsr *up = get_spin(m, 0, s->nup), *dn = get_spin(m, 1, s->ndn);
   for (SpinCsr *sp : {up, dn}) {
@@ -407,7 +386,6 @@ void ensure_ff(edgpu_model *m, Sector *s) {
       launch_pack_hops<ffloat>(sp->col.as<int>(), sp->vff.as<ffloat>(), sp->nnz, sp->uhff.as<Hop<ffloat>>(), c->stream);
     }
     if (sp->lv64.p && !sp->lvff.p) conv(sp->lvff, sp->lv64, (long long)std::max(1, sp->kmax) * sp->ld);
-    if (sp->vd_cells && !sp->vd_vff.p) conv(sp->vd_vff, sp->vd_v64, sp->vd_cells);
   }
   conv(s->diagff, s->diag64, s->dim);
   const SectorOp<double> &d = s->op64;
@@ -458,12 +436,9 @@ void ensure_ff(edgpu_model *m, Sector *s) {
   o.M_ = nullptr;
   o.M_val = nullptr;
   o.nW = d.nW;
-  o.kW = d.kW;
   o.vu_cnt = d.vu_cnt;
   o.vu_ent = d.vu_ent;
-  o.vd_len = d.vd_len;
-  o.vd_col = d.vd_col;
-  o.vd_val = dn->vd_vff.as<ffloat>();
+  o.vd_to = d.vd_to;
   s->dopff = DBuf(c->alloc, sizeof(SectorOp<ffloat>));
   CK(cudaMemcpyAsync(s->dopff.p, &s->opff, sizeof(SectorOp<ffloat>), cudaMemcpyHostToDevice, c->stream));
   sync(c);
@@ -515,18 +490,13 @@ Sector *get_sector(edgpu_model *m, int storage, int nup, int ndn) {
     s->op32.up_hop = up->uh32.as<Hop<float>>();
     s->op64.dn_slot = dn->slot2.as<unsigned short>();
     s->op32.dn_slot = dn->slot4.as<unsigned short>();
-    s->op64.nV = s->op32.nV = (int)m->Vs.size();
-    s->op64.V_ = s->op32.V_ = m->dVs.as<Transition>();
-    s->op64.V_val = m->dVsv64.as<double>();
-    s->op32.V_val = m->dVsv32.as<float>();
-    s->op64.nW = s->op32.nW = m->vprod.dev.nW;
-    s->op64.kW = s->op32.kW = m->vprod.dev.kW;
-    s->op64.vu_cnt = s->op32.vu_cnt = up->vu_cnt.as<int>();
-    s->op64.vu_ent = s->op32.vu_ent = up->vu_ent.as<int2>();
-    s->op64.vd_len = s->op32.vd_len = dn->vd_len.as<int>();
-    s->op64.vd_col = s->op32.vd_col = dn->vd_col.as<int>();
-    s->op64.vd_val = dn->vd_v64.as<double>();
-    s->op32.vd_val = dn->vd_v32.as<float>();
+    if (m->vprod.dev.nW > 0) {
+      s->op64.nV = s->op32.nV = 0;
+      s->op64.nW = s->op32.nW = m->vprod.dev.nW;
+      s->op64.vu_cnt = s->op32.vu_cnt = up->vu_cnt.as<int>();
+      s->op64.vu_ent = s->op32.vu_ent = up->vu_ent.as<int4>();
+      s->op64.vd_to = s->op32.vd_to = dn->vd_to.as<int>();
+    }
     if (s->dim > (long long)INT_MAX)
       throw ApiError(EDGPU_ERR_CAPACITY, "spin-resolved sector above 2^31 - 1 states");
     if (srs_two_pass(s->up_rows, s->dn_rows)) {

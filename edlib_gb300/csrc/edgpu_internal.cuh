@@ -230,31 +230,29 @@ struct SectorOp {
   // tables for state <-> index and matrix-free transitions
   const int *up_basis, *dn_basis;    // masks of the C(Ns,N) states
   const int *ninv_up, *ninv_dn;      // ninv rows for N_up, N_dn
-  int nT, nV;                        // SRS: V_ holds the interaction terms outside the product tables below
+  int nT, nV;                        // SRS: nV = 0 where the product tables below hold the interaction
   const Transition *T_;
   const Transition *V_;
   const T *T_val;                    // transition values in vector precision
   const T *V_val;
-  // SRS: interaction terms between the spins as sum_h A_h (x) W_h (host::VProd): up row u has vu_cnt[u] entries
-  // {source row, h << 1 | negative} at vu_ent[u * nW + e]; W_h k-major over the down rows, entry k of row d at
-  // [(h * kW + k) * dn_ld + d], lengths vd_len[h * dn_ld + d]
   // SOCRS: every transition (T and V) as masks, values with the constant part of the sign
   int nM;
   const TransMask *M_;
   const T *M_val;
-  int nW, kW;
+  // SRS: the interaction terms c+_i c+_j c_l c_k, all between the spins, by their one-spin halves (host::VProd): up row u
+  // has vu_cnt[u] entries {source row, down hop g, term, negative} at vu_ent[u * nW + e], in the order of the terms; down
+  // hop g takes row d to vd_to[g * dn_ld + d] = target << 1 | negative, or -1
+  int nW;
   const int *vu_cnt;
-  const int2 *vu_ent;
-  const int *vd_len, *vd_col;
-  const T *vd_val;
+  const int4 *vu_ent;
+  const int *vd_to;
 };
 
-// The interaction terms between the spins of a model as products of one-spin hops: distinct up hops c+_I c_K
-// (upI, upK), h = 0 .. nW - 1, each with its down hops c+_J c_L and values at [off[h], off[h + 1]).
+// The interaction terms of a model as pairs of one-spin hops: term q (0 .. nW - 1) is number t[q] of the model's, its up half
+// c+_upI c_upK, its down half number g[q] of the distinct hops c+_dnJ c_dnL (0 .. ng - 1).
 struct DevVProd {
-  int nW, kW;
-  const int *upI, *upK, *off, *dnJ, *dnL;
-  const double *val;
+  int nW, ng;
+  const int *upI, *upK, *g, *t, *dnJ, *dnL;
 };
 
 template <typename T>

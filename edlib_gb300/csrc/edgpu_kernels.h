@@ -90,12 +90,12 @@ void launch_spin_csr(const DevModel &m, int spin, int k, long long rows, const i
 // k-major ("ELL") copy of a per-spin CSR: len[d], col/val[k * ld + d]; the padding stays as memset (0)
 void launch_spin_ell(const int *rp, const int *col, const double *v64, const float *v32, int rows, int ld, int *len,
                      int *ell_col, double *ell_v64, float *ell_v32, cudaStream_t st);
-// one-spin halves of the product interaction terms: up entries of the rows with k up electrons, and the down
-// matrices W_h of the rows with k down electrons (SectorOp::vu_*, vd_*; vd_len and values past it stay as memset)
-void launch_vprod_up(const DevModel &m, const DevVProd &vp, int k, int rows, const int *basis_k, int *cnt, int2 *ent,
+// one-spin halves of the product interaction terms: up entries of the rows with k up electrons, and the down hops of the
+// rows with k down electrons (SectorOp::vu_*, vd_to)
+void launch_vprod_up(const DevModel &m, const DevVProd &vp, int k, int rows, const int *basis_k, int *cnt, int4 *ent,
                      cudaStream_t st);
-void launch_vprod_dn(const DevModel &m, const DevVProd &vp, int k, int rows, int ld, const int *basis_k, int *len,
-                     int *col, double *v64, float *v32, cudaStream_t st);
+void launch_vprod_dn(const DevModel &m, const DevVProd &vp, int k, int rows, int ld, const int *basis_k, int *to,
+                     cudaStream_t st);
 // (column, value) pairs of n table entries
 template <typename T>
 void launch_pack_hops(const int *col, const T *val, long long n, Hop<T> *out, cudaStream_t st);

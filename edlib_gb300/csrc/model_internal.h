@@ -83,15 +83,13 @@ struct DBuf {
   template <typename T> T *as() const { return reinterpret_cast<T *>(p); }
 };
 
-// The interaction terms of a spin-resolved operator.  A term c+_i c+_j c_l c_k whose two halves (k -> i, l -> j) act
-// on different spins is a product of one hop per spin, its signs the product of the two one-spin signs (each half
-// passes the other spin's electrons an even number of times); terms with the same up hop share one down matrix.
-// The others (both halves in one spin) stay in a transition list.
+// The interaction terms of a spin-resolved operator where each acts on both spins: a term c+_i c+_j c_l c_k whose two halves
+// (k -> i, l -> j) act on different spins is a product of one hop per spin, its sign the product of the two one-spin signs
+// (each half passes the other spin's electrons an even number of times).  Terms stay apart and in the model's order, in
+// which every element sums them.
 struct VProd {
-  std::vector<int> upI, upK, off, dnJ, dnL;
-  std::vector<double> val;
-  int kW = 0;  // most down hops of one up hop
-  DBuf dI, dK, doff, dJ, dL, dval;
+  std::vector<int> upI, upK, g, t, dnJ, dnL;
+  DBuf dI, dK, dg, dt, dJ, dL;
   DevVProd dev{};
 };
 
@@ -108,8 +106,7 @@ struct SpinCsr {
   DBuf vff, ell_vff;                     // float-float values (built on first use, ensure_ff)
   std::vector<int> hrp;            // host copy of the row pointers
   DBuf vu_cnt, vu_ent;             // up spin: entries of the product interaction terms (SectorOp::vu_*)
-  DBuf vd_len, vd_col, vd_v64, vd_v32, vd_vff;  // down spin: their down matrices (SectorOp::vd_*)
-  long long vd_cells = 0;
+  DBuf vd_to;                      // down spin: their down hops (SectorOp::vd_to)
 };
 
 struct Sector {
@@ -161,8 +158,6 @@ struct edgpu_model {
   double mu = 0;
   size_t max_dim = 0, max_size = 0;
   edgpu::host::DBuf dTvff, dVvff;  // float-float transition values (ensure_ff)
-  std::vector<edgpu::Transition> Vs;  // interaction terms of the spin-resolved operator outside the product tables
-  edgpu::host::DBuf dVs, dVsv64, dVsv32;
   edgpu::host::DBuf dM, dMv64, dMv32;  // every transition as masks (SectorOp::M_)
   edgpu::host::VProd vprod;
   edgpu::host::DBuf dT, dV, dTv64, dTv32, dVv64, dVv32, dU, dxmu, dhmag, dJ, depsk, dh0, dUt, dbinom, dbasis, dninv;

@@ -56,41 +56,40 @@ struct RowPart {
   T v[C];
 };
 
-// Off-diagonal interaction of C elements of an SRS row, columns d0, d0 + S, ... (those below Nd), added to a: the
-// product terms from the one-spin tables -- per up entry of the row (source row, h) the entries of W_h in each
-// column -- then the terms listed as transitions.  A Kanamori impurity has about one up entry per row and one entry
-// per column of W_h, where testing every transition on every state cost 24 state tests with two rank lookups per
-// hit: the 12-orbital Kanamori sector (6,6), four FP32 vectors, went from 866 to 78 us.  (Not inlined: models without
-// such terms keep the registers.)
+// Off-diagonal interaction of C elements of an SRS row, columns d0, d0 + S, ... (those below Nd), added to a in the order of
+// the terms: each up entry of the row (source row, down hop, term) by the entry of the down hop in each column, or, for a
+// model without these tables, the transitions.  A Kanamori impurity has about four up entries per row, one in four of which
+// meets a down hop of a column, where testing every transition on every state cost 24 state tests with two rank lookups
+// per hit.  (Not inlined: models without such terms keep the registers.)
 template <typename T, int C, int S>
 __device__ __noinline__ RowPart<T, C> srs_vloc(const SectorOp<T> *opp, int u, int d0, const T *__restrict__ x, RowPart<T, C> a) {
   const SectorOp<T> &op = *opp;
-  const int Nd = op.dn_rows;
-  const int ne = op.nW ? ldg_t(op.vu_cnt + u) : 0;
-  for (int e = 0; e < ne; ++e) {
-    const int2 en = __ldg(op.vu_ent + (long long)u * op.nW + e);
-    const int h = en.y >> 1;
-    const T *__restrict__ xr = x + (long long)en.x * Nd;
-    int len[C], kk = 0;
+  constexpr int U = 4;  // entries in flight
+  const int Nd = op.dn_rows, ne = op.nW ? ldg_t(op.vu_cnt + u) : 0;
+  for (int e = 0; e < ne; e += U) {
+    int4 en[U];
+    int to[U][C];
+    T v[U], xv[U][C];
 #pragma unroll
-    for (int cc = 0; cc < C; ++cc) {
-      len[cc] = d0 + cc * S < Nd ? ldg_t(op.vd_len + h * op.dn_ld + d0 + cc * S) : 0;
-      kk = max(kk, len[cc]);
+    for (int q = 0; q < U; ++q) en[q] = e + q < ne ? __ldg(op.vu_ent + (long long)u * op.nW + e + q) : make_int4(0, 0, -1, 0);
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      const bool in = en[q].z >= 0;
+      v[q] = in ? ldg_t(op.V_val + en[q].z) : T(0);
+      if (en[q].w) v[q] = -v[q];
+#pragma unroll
+      for (int cc = 0; cc < C; ++cc) to[q][cc] = in && d0 + cc * S < Nd ? ldg_t(op.vd_to + en[q].y * op.dn_ld + d0 + cc * S) : -1;
     }
-    for (int k = 0; k < kk; ++k) {
-      const int o = (h * op.kW + k) * op.dn_ld + d0;
-      T v[C], xv[C];
 #pragma unroll
-      for (int cc = 0; cc < C; ++cc) {
-        const bool in = k < len[cc];
-        v[cc] = in ? ldg_t(op.vd_val + o + cc * S) : T(0);
-        xv[cc] = in ? ldg_t(xr + ldg_t(op.vd_col + o + cc * S)) : T(0);
-        if (en.y & 1) v[cc] = -v[cc];
-      }
+    for (int q = 0; q < U; ++q)
 #pragma unroll
       for (int cc = 0; cc < C; ++cc)
-        if (k < len[cc]) a.v[cc] += v[cc] * xv[cc];
-    }
+        xv[q][cc] = to[q][cc] >= 0 ? ldg_t(x + (long long)en[q].x * Nd + (to[q][cc] >> 1)) : T(0);
+#pragma unroll
+    for (int q = 0; q < U; ++q)
+#pragma unroll
+      for (int cc = 0; cc < C; ++cc)
+        if (to[q][cc] >= 0) a.v[cc] = madd(to[q][cc] & 1 ? -v[q] : v[q], xv[q][cc], a.v[cc]);
   }
   if (op.nV) {
     for (int cc = 0; cc < C; ++cc)
@@ -114,36 +113,41 @@ template <typename T, int R>
 __device__ __noinline__ RowPart<T, R> srs_vloc_rows(const SectorOp<T> *opp, int u, int nr, int d, const T *__restrict__ x,
                                                     RowPart<T, R> a) {
   const SectorOp<T> &op = *opp;
+  constexpr int U = 2;
   int ne[R], nmax = 0;
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     ne[r] = op.nW && r < nr ? ldg_t(op.vu_cnt + u + r) : 0;
     nmax = max(nmax, ne[r]);
   }
-  for (int e = 0; e < nmax; ++e) {
-    int2 en[R];
-    int len[R], kk = 0;
+  for (int e = 0; e < nmax; e += U) {
+    int4 en[U][R];
+    int to[U][R];
+    T v[U][R], xv[U][R];
 #pragma unroll
-    for (int r = 0; r < R; ++r) en[r] = e < ne[r] ? __ldg(op.vu_ent + (long long)(u + r) * op.nW + e) : make_int2(0, 0);
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      len[r] = e < ne[r] ? ldg_t(op.vd_len + (en[r].y >> 1) * op.dn_ld + d) : 0;
-      kk = max(kk, len[r]);
-    }
-    for (int k = 0; k < kk; ++k) {
-      T v[R], xv[R];
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const bool in = k < len[r];
-        const int o = ((en[r].y >> 1) * op.kW + k) * op.dn_ld + d;
-        v[r] = in ? ldg_t(op.vd_val + o) : T(0);
-        xv[r] = in ? ldg_t(x + (long long)en[r].x * op.dn_rows + ldg_t(op.vd_col + o)) : T(0);
-        if (en[r].y & 1) v[r] = -v[r];
-      }
+    for (int q = 0; q < U; ++q)
 #pragma unroll
       for (int r = 0; r < R; ++r)
-        if (k < len[r]) a.v[r] += v[r] * xv[r];
-    }
+        en[q][r] = e + q < ne[r] ? __ldg(op.vu_ent + (long long)(u + r) * op.nW + e + q) : make_int4(0, 0, -1, 0);
+#pragma unroll
+    for (int q = 0; q < U; ++q)
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const bool in = en[q][r].z >= 0;
+        v[q][r] = in ? ldg_t(op.V_val + en[q][r].z) : T(0);
+        to[q][r] = in ? ldg_t(op.vd_to + en[q][r].y * op.dn_ld + d) : -1;
+        if ((en[q][r].w ^ to[q][r]) & 1) v[q][r] = -v[q][r];
+      }
+#pragma unroll
+    for (int q = 0; q < U; ++q)
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        xv[q][r] = to[q][r] >= 0 ? ldg_t(x + (long long)en[q][r].x * op.dn_rows + (to[q][r] >> 1)) : T(0);
+#pragma unroll
+    for (int q = 0; q < U; ++q)
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (to[q][r] >= 0) a.v[r] = madd(v[q][r], xv[q][r], a.v[r]);
   }
   if (op.nV) {
     for (int r = 0; r < nr; ++r) {

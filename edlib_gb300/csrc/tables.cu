@@ -393,44 +393,36 @@ __device__ inline bool spin_hop(int ns, int mask, int I, int K, int &to, int &si
   return true;
 }
 
-__global__ void k_vprod_up(DevModel m, DevVProd vp, int k, int rows, const int *basis_k, int *cnt, int2 *ent) {
+__global__ void k_vprod_up(DevModel m, DevVProd vp, int k, int rows, const int *basis_k, int *cnt, int4 *ent) {
   for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < rows; u += gridDim.x * blockDim.x) {
     int n = 0;
-    for (int h = 0; h < vp.nW; ++h) {
+    for (int q = 0; q < vp.nW; ++q) {
       int to, sign;
-      if (!spin_hop(m.ns, basis_k[u], vp.upI[h], vp.upK[h], to, sign)) continue;
-      ent[(long long)u * vp.nW + n++] = make_int2(m.ninv[((long long)k << m.ns) | to], h << 1 | (sign < 0 ? 1 : 0));
+      if (!spin_hop(m.ns, basis_k[u], vp.upI[q], vp.upK[q], to, sign)) continue;
+      ent[(long long)u * vp.nW + n++] = make_int4(m.ninv[((long long)k << m.ns) | to], vp.g[q], vp.t[q], sign < 0);
     }
     cnt[u] = n;
   }
 }
 
-__global__ void k_vprod_dn(DevModel m, DevVProd vp, int k, int rows, int ld, const int *basis_k, int *len, int *col,
-                           double *v64, float *v32) {
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < rows * vp.nW; t += gridDim.x * blockDim.x) {
-    const int h = t / rows, d = t - h * rows;
-    int n = 0;
-    for (int q = vp.off[h]; q < vp.off[h + 1]; ++q) {
-      int to, sign;
-      if (!spin_hop(m.ns, basis_k[d], vp.dnJ[q], vp.dnL[q], to, sign)) continue;
-      const long long e = ((long long)h * vp.kW + n++) * ld + d;
-      col[e] = m.ninv[((long long)k << m.ns) | to];
-      v64[e] = sign * vp.val[q];
-      v32[e] = (float)(sign * vp.val[q]);
-    }
-    len[h * ld + d] = n;
+__global__ void k_vprod_dn(DevModel m, DevVProd vp, int k, int rows, int ld, const int *basis_k, int *to_) {
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < rows * vp.ng; t += gridDim.x * blockDim.x) {
+    const int g = t / rows, d = t - g * rows;
+    int to, sign;
+    const bool ok = spin_hop(m.ns, basis_k[d], vp.dnJ[g], vp.dnL[g], to, sign);
+    to_[g * ld + d] = ok ? m.ninv[((long long)k << m.ns) | to] << 1 | (sign < 0 ? 1 : 0) : -1;
   }
 }
 
-void launch_vprod_up(const DevModel &m, const DevVProd &vp, int k, int rows, const int *basis_k, int *cnt, int2 *ent,
+void launch_vprod_up(const DevModel &m, const DevVProd &vp, int k, int rows, const int *basis_k, int *cnt, int4 *ent,
                      cudaStream_t st) {
   k_vprod_up<<<std::max(1, std::min(1024, (rows + 127) / 128)), 128, 0, st>>>(m, vp, k, rows, basis_k, cnt, ent); note_launch();
 }
 
-void launch_vprod_dn(const DevModel &m, const DevVProd &vp, int k, int rows, int ld, const int *basis_k, int *len,
-                     int *col, double *v64, float *v32, cudaStream_t st) {
-  const int n = rows * vp.nW;
-  k_vprod_dn<<<std::max(1, std::min(1024, (n + 127) / 128)), 128, 0, st>>>(m, vp, k, rows, ld, basis_k, len, col, v64, v32); note_launch();
+void launch_vprod_dn(const DevModel &m, const DevVProd &vp, int k, int rows, int ld, const int *basis_k, int *to,
+                     cudaStream_t st) {
+  const int n = rows * vp.ng;
+  k_vprod_dn<<<std::max(1, std::min(1024, (n + 127) / 128)), 128, 0, st>>>(m, vp, k, rows, ld, basis_k, to); note_launch();
 }
 
 void launch_spin_ell(const int *rp, const int *col, const double *v64, const float *v32, int rows, int ld, int *len,
