@@ -795,63 +795,99 @@ __device__ __noinline__ DotAcc srs_flat(const SrsItem<T> &it, const ItemHops<T> 
   return acc;
 }
 
-// Sum over the L lanes (a power of two) of a row, in every one of them.
-template <typename T, int L>
-__device__ __forceinline__ T row_sum(T v) {
-#pragma unroll
-  for (int o = L / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
+// lanes that share a row of the CRS and the SOCRS storage
+template <int ST>
+constexpr int kRowLanes = ST == kCRS ? 4 : 8;
 
-// One item of a sector (CRS, SOCRS): y[lo:hi) = (H x)[lo:hi) + c z[lo:hi); the thread's part of <x, y>.  L lanes share
-// a row and add their parts by a fixed butterfly.  CRS: lane q takes the row's entries q, q + L, ..., so that a row's
-// values and columns are read side by side and its x loads are in flight at once; with one thread per row each waited
-// for its own chain of loads (4900 rows of 17 entries, one FP64 vector: 27 -> 7 us cold).  SOCRS: lane q takes
-// transitions q, q + L, ..., each a test of masks (TransMask; 52,920 rows of 36 transitions, two FP64 vectors:
-// 91 -> 38 us, the rows' own 64-bit decoding of every transition before).
+// One item of a sector: y[lo:hi) = (H x)[lo:hi) + c z[lo:hi); the thread's part of <x, y>.  L lanes share a row: they read
+// its entries side by side, and each adds all of them in the row's order, handed around by shuffles, so that the sum is
+// that of one thread per row.  CRS: lane q reads entries q, q + L, ... of the row, U rounds of them in flight; one thread
+// per row waited for its own chain of loads (4900 rows of 17 entries, one FP64 vector: 27 us cold).  SOCRS: lane q tests
+// transitions q, q + L, ... by masks (TransMask) and reads the elements they lead to (52,920 rows of 36 transitions, two
+// FP64 vectors: 91 us with the rows' own 64-bit decoding of every transition).
+// <x, y> is summed as with one thread per row too: lane q of a row group takes the rows of passes q, q + L, ..., which are
+// those of thread (row group) + (kMvBlock / L) q (row_dot).
 template <typename T, int ST>
 __device__ __forceinline__ DotAcc mv_item(const SectorOp<T> *opp, int rows, long long li, const T *__restrict__ x,
                                           T *__restrict__ y, const T *z, T c, bool want_dot) {
-  constexpr int L = ST == kCRS ? 4 : 8;
+  constexpr int L = kRowLanes<ST>;
   const SectorOp<T> &op = *opp;
   long long lo, hi;
   item_range(op, rows, li, lo, hi);
   const int q = threadIdx.x % L;
+  const unsigned lane0 = (threadIdx.x & 31) - q, group = ((1u << L) - 1) << lane0;
   DotAcc acc;
   dot_init(acc);
-  for (long long r0 = lo + threadIdx.x / L; r0 - threadIdx.x / L < hi; r0 += kMvBlock / L) {  // whole warps stay together
-    const bool in = r0 < hi;
-    const long long i = in ? r0 : hi - 1;
-    T v = T(0);
+  int pass = 0;
+  for (long long i = lo + threadIdx.x / L; i < hi; i += kMvBlock / L, ++pass) {  // a row's lanes stay together
+    T v;
     if constexpr (ST == kCRS) {
+      constexpr int U = 4;
       const long long j1 = op.crs_rp[i + 1];
-#pragma unroll 4
-      for (long long j = op.crs_rp[i] + q; j < j1; j += L) v += ldg_t(op.crs_val + j) * x[__ldg(op.crs_col + j)];
+      v = z ? mul_rn(c, z[i]) : T(0);
+      for (long long j = op.crs_rp[i] + q; j - q < j1; j += U * L) {
+        T a[U], b[U];
+#pragma unroll
+        for (int k = 0; k < U; ++k) {
+          const bool in = j + k * L < j1;
+          a[k] = in ? ldg_t(op.crs_val + j + k * L) : T(0);
+          b[k] = in ? x[__ldg(op.crs_col + j + k * L)] : T(0);
+        }
+#pragma unroll
+        for (int k = 0; k < U; ++k)
+#pragma unroll
+          for (int p = 0; p < L; ++p) {
+            const T av = __shfl_sync(group, a[k], p, L), bv = __shfl_sync(group, b[k], p, L);
+            if (j - q + k * L + p < j1) v = madd(av, bv, v);
+          }
+      }
     } else {
       const unsigned Nd = (unsigned)op.dn_rows;
       const long long u = op.dim <= 0xffffffffll ? (unsigned)i / Nd : i / Nd;
       const unsigned d = (unsigned)(i - u * Nd);
       const unsigned long long s = ((unsigned long long)__ldg(op.up_basis + u) << op.ns) | (unsigned)__ldg(op.dn_basis + d);
+      v = mul_rn(ldg_t(op.diag + i), x[i]);
+      if (z) v = madd(c, z[i], v);
 #pragma unroll 2
-      for (int k = q; k < op.nM; k += L) {
-        const ulonglong2 a = __ldg(reinterpret_cast<const ulonglong2 *>(op.M_ + k));
-        if ((s & a.y) != a.x) continue;
-        const ulonglong2 b = __ldg(reinterpret_cast<const ulonglong2 *>(op.M_ + k) + 1);
-        const unsigned long long t = s ^ b.x;
-        const long long col = (long long)__ldg(op.ninv_up + (t >> op.ns)) * Nd + __ldg(op.ninv_dn + (t & ((1ull << op.ns) - 1)));
-        const T m = ldg_t(op.M_val + k);
-        v += (__popcll(s & b.y) & 1 ? -m : m) * x[col];
+      for (int k0 = 0; k0 < op.nM; k0 += L) {
+        const int k = k0 + q;
+        T m = T(0), b = T(0);
+        bool hit = false;
+        if (k < op.nM) {
+          const ulonglong2 a = __ldg(reinterpret_cast<const ulonglong2 *>(op.M_ + k));
+          hit = (s & a.y) == a.x;
+          if (hit) {
+            const ulonglong2 f = __ldg(reinterpret_cast<const ulonglong2 *>(op.M_ + k) + 1);
+            const unsigned long long t = s ^ f.x;
+            const long long col = (long long)__ldg(op.ninv_up + (t >> op.ns)) * Nd + __ldg(op.ninv_dn + (t & ((1ull << op.ns) - 1)));
+            m = ldg_t(op.M_val + k);
+            if (__popcll(s & f.y) & 1) m = -m;
+            b = x[col];
+          }
+        }
+        for (unsigned h = __ballot_sync(group, hit) >> lane0; h; h &= h - 1) {
+          const int p = __ffs(h) - 1;
+          v = madd(__shfl_sync(group, m, p, L), __shfl_sync(group, b, p, L), v);
+        }
       }
     }
-    v = row_sum<T, L>(v);
-    if (in && q == 0) {
-      if constexpr (ST == kSOCRS) v += ldg_t(op.diag + i) * x[i];
-      if (z) v = v + c * z[i];
-      y[i] = v;
-      if (want_dot) dot_add(acc, x[i], v);
-    }
+    if (q == 0) y[i] = v;
+    if (want_dot && pass % L == q) dot_add(acc, x[i], v);
   }
   return acc;
+}
+
+// mv_item's parts of <x, y> to the threads whose sums they are
+template <typename T, int ST>
+__device__ __forceinline__ DotAcc row_dot(const DotAcc &acc, double *part) {
+  constexpr int L = kRowLanes<ST>;
+  __syncthreads();
+  part[threadIdx.x / L + kMvBlock / L * (threadIdx.x % L)] = dot_value(acc);
+  __syncthreads();
+  DotAcc r;
+  dot_init(r);
+  r.d = part[threadIdx.x];
+  return r;
 }
 
 // <x, y> of an item into its recurrence's parts; the block that finishes the task's last item sums them: alf.
@@ -1197,12 +1233,17 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_srs_long(Src src, int nitems)
 // CRS and SOCRS items
 template <typename T, class Src, int ST>
 __global__ void __launch_bounds__(kMvBlock, 3) k_row_mv(Src src, int nitems) {
-  __shared__ double red[kMvBlock / 32];
+  __shared__ double red[kMvBlock / 32], part[Src::kEarly ? kMvBlock : 1];
   if constexpr (Src::kEarly) pdl_enter();
   for (int i = blockIdx.x; i < nitems; i += gridDim.x)
     src.get(i, [&](const SectorOp<T> *op, int rows, int li, const T *x, T *y, const T *z, T c, const LzTask<T> *lz) {
       DotAcc acc = mv_item<T, ST>(op, rows, li, x, y, z, c, lz != nullptr);
-      if (lz) emit_dot<T, kMvBlock>(*lz, acc, lz->part_a + li, red);
+      if constexpr (Src::kEarly) {
+        if (lz) {
+          acc = row_dot<T, ST>(acc, part);
+          emit_dot<T, kMvBlock>(*lz, acc, lz->part_a + li, red);
+        }
+      }
     });
 }
 
