@@ -231,8 +231,22 @@ struct LzTask {
   double *part_a;     // [nitems]
   double *part_b;     // [nitems]
   double *scal;       // [0] alf, [1] bet
-  int *state;         // [0] done, [1] nlanc, [2] items of the operator done in this step, [3] of the alpha pass
+  int *state;         // [0] done, [1] nlanc, [2] items whose <v, w> is done in this step, [3] of the alpha pass
   int nlanc_max;
+  int mv_rows;        // rows per item and first item of the product, where it has items of its own (LzBatch::split)
+  int mv_begin;
+};
+
+// A batch of recurrences for launch_lz_step.  split: the product has its own, smaller items (mv_items of them) and <v, w>
+// a pass of its own over the recurrences' items, which are too few where rows are short or stored row by row.
+template <typename T>
+struct LzBatch {
+  const LzTask<T> *tasks;
+  const int *item_task;
+  int nitems;
+  bool split = false;
+  const int *mv_item_task = nullptr;
+  int mv_items = 0;
 };
 
 // Restarted Lanczos eigen-solver task with full classical Gram-Schmidt (twice).
@@ -344,8 +358,7 @@ void launch_wait_selftest(int rounds, int *gave_up_dev, cudaStream_t st);
 // true (and cleared) when a bounded wait of the Gram-Schmidt dot pass gave up on a bulk copy
 bool take_cgs_stall();
 template <typename T>
-void launch_lz_mv(const LzTask<T> *tasks_dev, const int *item_task_dev, int nitems_total, int it, bool early, MvShape sh,
-                  cudaStream_t st);
+void launch_lz_mv(const LzBatch<T> &b, int it, bool early, MvShape sh, cudaStream_t st);
 template <typename T>
 void launch_eig_mv(const EigTask<T> *tasks_dev, const int *item_task_dev, int nitems_total, MvShape sh, cudaStream_t st,
                    T *probe_y = nullptr);
@@ -355,8 +368,7 @@ template <typename T>
 OpTuning tune_eig_mv(const EigTask<T> *tasks_dev, const int *item_task_dev, int nitems_total, MvShape sh, T *probe_y,
                      cudaStream_t st);
 template <typename T>
-void launch_lz_step(const LzTask<T> *tasks_dev, const int *item_task_dev, int nitems_total, int it, MvShape sh,
-                    cudaStream_t st);
+void launch_lz_step(const LzBatch<T> &b, int it, MvShape sh, cudaStream_t st);
 // Kernel attributes the step kernels need for this shape; call before launch_eig_step (and before a
 // step is captured into a graph).
 template <typename T>

@@ -178,9 +178,8 @@ void run_lanczos_ff(edgpu_model *m, std::vector<LzJob<double> *> &jobs, int nlan
     merge_shape(shape, mv_shape<double>(s, true));  // float-float elements take the room of FP64 ones
   }
   DBuf dt = upload(c, tasks), dm = upload(c, item_task);
-  for (int it = 0; it < nlanc; ++it)
-    launch_lz_step<ffloat>(dt.as<LzTask<ffloat>>(), dm.as<int>(), (int)item_task.size(), it, shape,
-                           c->stream);
+  const LzBatch<ffloat> batch{dt.as<LzTask<ffloat>>(), dm.as<int>(), (int)item_task.size()};
+  for (int it = 0; it < nlanc; ++it) launch_lz_step<ffloat>(batch, it, shape, c->stream);
   CK(cudaGetLastError());
   sync(c);
   trace_coefficients(jobs, nlanc, "ff");
@@ -204,7 +203,9 @@ void run_lanczos(edgpu_model *m, std::vector<LzJob<T> *> &jobs, int nlanc, bool 
     }
   }
   std::vector<LzTask<T>> tasks(jobs.size());
-  std::vector<int> item_task;
+  std::vector<int> item_task, mv_item_task;
+  bool split = true;  // only rows that are short or stored row by row: items of 2048 elements, a handful per recurrence
+  for (auto *J : jobs) split = split && (J->s->storage != kSRS || J->s->dn_rows < kSrsLongRow);
   MvShape shape{jobs[0]->s->storage, 0};
   for (size_t q = 0; q < jobs.size(); ++q) {
     LzJob<T> &J = *jobs[q];
@@ -233,11 +234,17 @@ void run_lanczos(edgpu_model *m, std::vector<LzJob<T> *> &jobs, int nlanc, bool 
     t.state = J.state.template as<int>();
     t.nlanc_max = nlanc;
     for (int it = 0; it < s.lz_nitems; ++it) item_task.push_back((int)q);
-    merge_shape(shape, mv_shape<T>(s, true));
+    if (split) {
+      t.mv_rows = s.srs_rows;
+      t.mv_begin = (int)mv_item_task.size();
+      for (int it = 0; it < s.nitems; ++it) mv_item_task.push_back((int)q);
+    }
+    merge_shape(shape, mv_shape<T>(s, !split));
   }
-  DBuf dt = upload(c, tasks), dm = upload(c, item_task);
-  for (int it = 0; it < nlanc; ++it)
-    launch_lz_step<T>(dt.template as<LzTask<T>>(), dm.template as<int>(), (int)item_task.size(), it, shape, c->stream);
+  DBuf dt = upload(c, tasks), dm = upload(c, item_task), dmv = upload(c, mv_item_task);
+  const LzBatch<T> batch{dt.template as<LzTask<T>>(), dm.template as<int>(), (int)item_task.size(), split,
+                         dmv.template as<int>(), (int)mv_item_task.size()};
+  for (int it = 0; it < nlanc; ++it) launch_lz_step<T>(batch, it, shape, c->stream);
   CK(cudaGetLastError());
   sync(c);
   trace_coefficients(jobs, nlanc, sizeof(T) == 8 ? "fp64" : "fp32");

@@ -795,36 +795,26 @@ __device__ __noinline__ DotAcc srs_flat(const SrsItem<T> &it, const ItemHops<T> 
   return acc;
 }
 
-// lanes that share a row of the CRS and the SOCRS storage
-template <int ST>
-constexpr int kRowLanes = ST == kCRS ? 4 : 8;
-
-// One item of a sector: y[lo:hi) = (H x)[lo:hi) + c z[lo:hi); the thread's part of <x, y>.  L lanes share a row: they read
-// its entries side by side, and each adds all of them in the row's order, handed around by shuffles, so that the sum is
-// that of one thread per row.  CRS: lane q reads entries q, q + L, ... of the row, U rounds of them in flight; one thread
-// per row waited for its own chain of loads (4900 rows of 17 entries, one FP64 vector: 27 us cold).  SOCRS: lane q tests
-// transitions q, q + L, ... by masks (TransMask) and reads the elements they lead to (52,920 rows of 36 transitions, two
-// FP64 vectors: 91 us with the rows' own 64-bit decoding of every transition).
-// <x, y> is summed as with one thread per row too: lane q of a row group takes the rows of passes q, q + L, ..., which are
-// those of thread (row group) + (kMvBlock / L) q (row_dot).
+// One item of a sector: y[lo:hi) = (H x)[lo:hi) + c z[lo:hi), every row added in its own order.  CRS: four lanes share a
+// row; they read its entries side by side, U rounds of them in flight, and each adds all of them, handed around by
+// shuffles.  (One thread per row waited for its own chain of loads: 4900 rows of 17 entries, one FP64 vector, 27 us cold
+// in three items of 2048 rows.)  SOCRS: a thread per row tests the transitions by their masks (TransMask), U of them with
+// their loads in flight; in FP64 one lane per row also keeps a warp's additions to one per transition, where eight lanes
+// per row (butterfly, or handed around in order) took eight times the FP64 issue slots.
 template <typename T, int ST>
-__device__ __forceinline__ DotAcc mv_item(const SectorOp<T> *opp, int rows, long long li, const T *__restrict__ x,
-                                          T *__restrict__ y, const T *z, T c, bool want_dot) {
-  constexpr int L = kRowLanes<ST>;
+__device__ __forceinline__ void mv_item(const SectorOp<T> *opp, int rows, long long li, const T *__restrict__ x,
+                                        T *__restrict__ y, const T *z, T c) {
   const SectorOp<T> &op = *opp;
+  constexpr int U = 4;
   long long lo, hi;
   item_range(op, rows, li, lo, hi);
-  const int q = threadIdx.x % L;
-  const unsigned lane0 = (threadIdx.x & 31) - q, group = ((1u << L) - 1) << lane0;
-  DotAcc acc;
-  dot_init(acc);
-  int pass = 0;
-  for (long long i = lo + threadIdx.x / L; i < hi; i += kMvBlock / L, ++pass) {  // a row's lanes stay together
-    T v;
-    if constexpr (ST == kCRS) {
-      constexpr int U = 4;
+  if constexpr (ST == kCRS) {
+    constexpr int L = 4;
+    const int q = threadIdx.x % L;
+    const unsigned group = ((1u << L) - 1) << ((threadIdx.x & 31) - q);
+    for (long long i = lo + threadIdx.x / L; i < hi; i += kMvBlock / L) {  // a row's lanes stay together
       const long long j1 = op.crs_rp[i + 1];
-      v = z ? mul_rn(c, z[i]) : T(0);
+      T v = z ? mul_rn(c, z[i]) : T(0);
       for (long long j = op.crs_rp[i] + q; j - q < j1; j += U * L) {
         T a[U], b[U];
 #pragma unroll
@@ -841,53 +831,39 @@ __device__ __forceinline__ DotAcc mv_item(const SectorOp<T> *opp, int rows, long
             if (j - q + k * L + p < j1) v = madd(av, bv, v);
           }
       }
-    } else {
-      const unsigned Nd = (unsigned)op.dn_rows;
+      if (q == 0) y[i] = v;
+    }
+  } else {
+    const unsigned Nd = (unsigned)op.dn_rows;
+    for (long long i = lo + threadIdx.x; i < hi; i += kMvBlock) {
       const long long u = op.dim <= 0xffffffffll ? (unsigned)i / Nd : i / Nd;
       const unsigned d = (unsigned)(i - u * Nd);
       const unsigned long long s = ((unsigned long long)__ldg(op.up_basis + u) << op.ns) | (unsigned)__ldg(op.dn_basis + d);
-      v = mul_rn(ldg_t(op.diag + i), x[i]);
+      T v = mul_rn(ldg_t(op.diag + i), x[i]);
       if (z) v = madd(c, z[i], v);
-#pragma unroll 2
-      for (int k0 = 0; k0 < op.nM; k0 += L) {
-        const int k = k0 + q;
-        T m = T(0), b = T(0);
-        bool hit = false;
-        if (k < op.nM) {
+      for (int k0 = 0; k0 < op.nM; k0 += U) {
+        T m[U], b[U];
+        bool hit[U];
+#pragma unroll
+        for (int p = 0; p < U; ++p) {
+          const int k = min(k0 + p, op.nM - 1);
           const ulonglong2 a = __ldg(reinterpret_cast<const ulonglong2 *>(op.M_ + k));
-          hit = (s & a.y) == a.x;
-          if (hit) {
-            const ulonglong2 f = __ldg(reinterpret_cast<const ulonglong2 *>(op.M_ + k) + 1);
-            const unsigned long long t = s ^ f.x;
-            const long long col = (long long)__ldg(op.ninv_up + (t >> op.ns)) * Nd + __ldg(op.ninv_dn + (t & ((1ull << op.ns) - 1)));
-            m = ldg_t(op.M_val + k);
-            if (__popcll(s & f.y) & 1) m = -m;
-            b = x[col];
-          }
+          const ulonglong2 f = __ldg(reinterpret_cast<const ulonglong2 *>(op.M_ + k) + 1);
+          hit[p] = k0 + p < op.nM && (s & a.y) == a.x;
+          const unsigned long long t = s ^ f.x;
+          m[p] = ldg_t(op.M_val + k);
+          if (__popcll(s & f.y) & 1) m[p] = -m[p];
+          b[p] = T(0);
+          if (hit[p])
+            b[p] = x[(long long)__ldg(op.ninv_up + (t >> op.ns)) * Nd + __ldg(op.ninv_dn + (t & ((1ull << op.ns) - 1)))];
         }
-        for (unsigned h = __ballot_sync(group, hit) >> lane0; h; h &= h - 1) {
-          const int p = __ffs(h) - 1;
-          v = madd(__shfl_sync(group, m, p, L), __shfl_sync(group, b, p, L), v);
-        }
+#pragma unroll
+        for (int p = 0; p < U; ++p)
+          if (hit[p]) v = madd(m[p], b[p], v);
       }
+      y[i] = v;
     }
-    if (q == 0) y[i] = v;
-    if (want_dot && pass % L == q) dot_add(acc, x[i], v);
   }
-  return acc;
-}
-
-// mv_item's parts of <x, y> to the threads whose sums they are
-template <typename T, int ST>
-__device__ __forceinline__ DotAcc row_dot(const DotAcc &acc, double *part) {
-  constexpr int L = kRowLanes<ST>;
-  __syncthreads();
-  part[threadIdx.x / L + kMvBlock / L * (threadIdx.x % L)] = dot_value(acc);
-  __syncthreads();
-  DotAcc r;
-  dot_init(r);
-  r.d = part[threadIdx.x];
-  return r;
 }
 
 // <x, y> of an item into its recurrence's parts; the block that finishes the task's last item sums them: alf.
@@ -938,8 +914,9 @@ struct VecSource {
 };
 
 // Lanczos recurrence, phase 1.  Iteration iter (0-based) of Lanczos.h:44-68: v = buf[iter % 3],
-// w = buf[(iter + 1) % 3] = H v - bet buf[(iter + 2) % 3]; a finished recurrence has nothing to do.
-template <typename T>
+// w = buf[(iter + 1) % 3] = H v - bet buf[(iter + 2) % 3], and <v, w> unless SPLIT (LzBatch); a finished recurrence has
+// nothing to do.
+template <typename T, bool SPLIT>
 struct LzSource {
   static constexpr bool kEarly = true;
   const LzTask<T> *tasks;
@@ -949,8 +926,8 @@ struct LzSource {
   __device__ __forceinline__ bool get(int it, F &&f) const {
     const LzTask<T> &t = tasks[item_task[it]];
     if (t.state[0]) return false;
-    f(t.op, t.srs_rows, it - t.item_begin, t.buf[iter % 3], t.buf[(iter + 1) % 3],
-      iter == 0 ? nullptr : t.buf[(iter + 2) % 3], (T)(-t.scal[1]), &t);
+    f(t.op, SPLIT ? t.mv_rows : t.srs_rows, it - (SPLIT ? t.mv_begin : t.item_begin), t.buf[iter % 3], t.buf[(iter + 1) % 3],
+      iter == 0 ? nullptr : t.buf[(iter + 2) % 3], (T)(-t.scal[1]), SPLIT ? (const LzTask<T> *)nullptr : &t);
     return true;
   }
 };
@@ -1233,17 +1210,10 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_srs_long(Src src, int nitems)
 // CRS and SOCRS items
 template <typename T, class Src, int ST>
 __global__ void __launch_bounds__(kMvBlock, 3) k_row_mv(Src src, int nitems) {
-  __shared__ double red[kMvBlock / 32], part[Src::kEarly ? kMvBlock : 1];
   if constexpr (Src::kEarly) pdl_enter();
   for (int i = blockIdx.x; i < nitems; i += gridDim.x)
-    src.get(i, [&](const SectorOp<T> *op, int rows, int li, const T *x, T *y, const T *z, T c, const LzTask<T> *lz) {
-      DotAcc acc = mv_item<T, ST>(op, rows, li, x, y, z, c, lz != nullptr);
-      if constexpr (Src::kEarly) {
-        if (lz) {
-          acc = row_dot<T, ST>(acc, part);
-          emit_dot<T, kMvBlock>(*lz, acc, lz->part_a + li, red);
-        }
-      }
+    src.get(i, [&](const SectorOp<T> *op, int rows, int li, const T *x, T *y, const T *z, T c, const LzTask<T> *) {
+      mv_item<T, ST>(op, rows, li, x, y, z, c);
     });
 }
 
@@ -1327,7 +1297,7 @@ void launch_mv(const MvTask<T> *tasks_dev, const int *item_task_dev, int nitems_
   const MvSource<T> src{tasks_dev, item_task_dev};
   if (sh.storage != kSRS) launch_rows<T>(sh.storage, src, nitems_total, st);
   else if (sh.plain) launch_srs<T, MvSource<T>, false, false, kPlainHB<T>, kMvBlocks<T>>(src, nitems_total, sh, st);
-  else launch_srs<T, MvSource<T>, true, true, 1, kMvBlocks<T>>(src, nitems_total, sh, st);
+  else launch_srs<T, MvSource<T>, true, false, 1, kMvBlocks<T>>(src, nitems_total, sh, st);
 }
 
 template <typename T>
@@ -1340,16 +1310,17 @@ void launch_mv_vectors(const Sector_mv<T> &v, MvShape sh, cudaStream_t st) {
 }
 
 template <typename T>
-void launch_lz_mv(const LzTask<T> *tasks_dev, const int *item_task_dev, int nitems_total, int it, bool early, MvShape sh,
-                  cudaStream_t st) {
-  const LzSource<T> src{tasks_dev, item_task_dev, it};
-  if constexpr (!std::is_same<T, ffloat>::value) {  // float-float recurrences: spin-resolved storage only
-    if (sh.storage != kSRS) {
-      launch_rows<T>(sh.storage, src, nitems_total, st, early);
+void launch_lz_mv(const LzBatch<T> &b, int it, bool early, MvShape sh, cudaStream_t st) {
+  if constexpr (!std::is_same<T, ffloat>::value) {  // float-float recurrences: spin-resolved storage only, never split
+    if (b.split) {
+      const LzSource<T, true> src{b.tasks, b.mv_item_task, it};
+      if (sh.storage != kSRS) launch_rows<T>(sh.storage, src, b.mv_items, st, early);
+      else launch_srs<T, LzSource<T, true>, true, false, 1, kMvBlocks<T>>(src, b.mv_items, sh, st, early);
       return;
     }
   }
-  launch_srs<T, LzSource<T>, true, true, 1, kMvBlocks<T>>(src, nitems_total, sh, st, early);
+  const LzSource<T, false> src{b.tasks, b.item_task, it};
+  launch_srs<T, LzSource<T, false>, true, true, 1, kMvBlocks<T>>(src, b.nitems, sh, st, early);
 }
 
 // Kernel attributes of the eigen step's operator for a shape; called before a step is captured into a graph.

@@ -3,5 +3,5 @@
 
 namespace edgpu {
 
-template void launch_lz_mv<ffloat>(const LzTask<ffloat> *, const int *, int, int, bool, MvShape, cudaStream_t);
+template void launch_lz_mv<ffloat>(const LzBatch<ffloat> &, int, bool, MvShape, cudaStream_t);
 }  // namespace edgpu
