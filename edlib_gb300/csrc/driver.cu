@@ -178,21 +178,6 @@ void finish_model(edgpu_model *m) {
   m->dVv64 = upload(c, vv64);
   m->dVv32 = upload(c, vv32);
   split_interaction(m);
-  {
-    std::vector<TransMask> masks;
-    std::vector<double> v64;
-    std::vector<float> v32;
-    for (const auto *list : {&m->T, &m->V})
-      for (auto &t : *list) {
-        bool neg = false;
-        masks.push_back(trans_mask(t, m->ip, neg));
-        v64.push_back(neg ? -t.value : t.value);
-        v32.push_back((float)v64.back());
-      }
-    m->dM = upload(c, masks);
-    m->dMv64 = upload(c, v64);
-    m->dMv32 = upload(c, v32);
-  }
   std::vector<long long> binom((kMaxNs + 2) * (kMaxNs + 2), 0);
   for (int n = 0; n <= kMaxNs + 1; ++n)
     for (int k = 0; k <= n; ++k) binom[n * (kMaxNs + 2) + k] = binom_at_host(n, k);
@@ -329,6 +314,28 @@ static void ensure_long(edgpu_model *m, SpinCsr *s) {
   launch_order_values<double>(s->ell_v64.as<double>(), order.as<short>(), s->ld, km, s->lv64.as<double>(), c->stream);
 }
 
+// The transitions as masks for SOCRS products, T then V, and behind them their values (with the constant part of the sign)
+// in FP64 and in FP32; built with the model's first sector of that storage.  Returns their number.
+static size_t ensure_masks(edgpu_model *m) {
+  const size_t n = m->T.size() + m->V.size();
+  if (m->dM.p) return n;
+  std::vector<char> buf(n * (sizeof(TransMask) + sizeof(double) + sizeof(float)));
+  TransMask *mask = reinterpret_cast<TransMask *>(buf.data());
+  double *v64 = reinterpret_cast<double *>(mask + n);
+  float *v32 = reinterpret_cast<float *>(v64 + n);
+  size_t k = 0;
+  for (const auto *list : {&m->T, &m->V})
+    for (auto &t : *list) {
+      bool neg = false;
+      mask[k] = trans_mask(t, m->ip, neg);
+      v64[k] = neg ? -t.value : t.value;
+      v32[k] = (float)v64[k];
+      ++k;
+    }
+  m->dM = upload(m->ctx, buf);
+  return n;
+}
+
 template <typename T>
 void fill_common(edgpu_model *m, const Sector &s, SectorOp<T> &op, const T *diag, const T *tval, const T *vval) {
   op.storage = s.storage;
@@ -351,10 +358,9 @@ void fill_common(edgpu_model *m, const Sector &s, SectorOp<T> &op, const T *diag
   op.T_val = tval;
   op.V_val = vval;
   op.nW = 0;
-  op.nM = (int)(m->T.size() + m->V.size());
-  op.M_ = m->dM.as<TransMask>();
-  if constexpr (sizeof(T) == 4) op.M_val = m->dMv32.as<float>();
-  else op.M_val = m->dMv64.as<double>();
+  op.nM = 0;
+  op.M_ = nullptr;
+  op.M_val = nullptr;
   op.vu_cnt = op.vd_to = nullptr;
   op.vu_ent = nullptr;
   for (int q = 0; q < 2; ++q) {
@@ -542,6 +548,11 @@ Sector *get_sector(edgpu_model *m, int storage, int nup, int ndn) {
     s->op32.crs_val = s->crs_v32.as<float>();
   }
   if (storage == kSOCRS) {
+    const size_t nM = ensure_masks(m);
+    s->op64.nM = s->op32.nM = (int)nM;
+    s->op64.M_ = s->op32.M_ = m->dM.as<TransMask>();
+    s->op64.M_val = reinterpret_cast<const double *>(m->dM.as<TransMask>() + nM);
+    s->op32.M_val = reinterpret_cast<const float *>(s->op64.M_val + nM);
     DBuf err(c->alloc, sizeof(int));
     CK(cudaMemsetAsync(err.p, 0, sizeof(int), c->stream));
     launch_socrs_check(m->dm, s->op64, err.as<int>(), c->stream);

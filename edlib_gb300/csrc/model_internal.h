@@ -158,7 +158,7 @@ struct edgpu_model {
   double mu = 0;
   size_t max_dim = 0, max_size = 0;
   edgpu::host::DBuf dTvff, dVvff;  // float-float transition values (ensure_ff)
-  edgpu::host::DBuf dM, dMv64, dMv32;  // every transition as masks (SectorOp::M_)
+  edgpu::host::DBuf dM;  // every transition as masks, and their values (SectorOp::M_, M_val; ensure_masks)
   edgpu::host::VProd vprod;
   edgpu::host::DBuf dT, dV, dTv64, dTv32, dVv64, dVv32, dU, dxmu, dhmag, dJ, depsk, dh0, dUt, dbinom, dbasis, dninv;
   std::vector<long long> basis_off;
