@@ -167,14 +167,11 @@ void finish_model(edgpu_model *m) {
   edgpu_ctx *c = m->ctx;
   if (m->ns < 1 || m->ns > kMaxNs) throw ApiError(EDGPU_ERR_ARG, "NSITES must be in [1, 20]");
   m->ip = 2 * m->ns;
-  std::vector<double> tv64, vv64;
-  std::vector<float> tv32, vv32;
-  for (auto &t : m->T) { tv64.push_back(t.value); tv32.push_back((float)t.value); }
+  std::vector<double> vv64;
+  std::vector<float> vv32;
   for (auto &t : m->V) { vv64.push_back(t.value); vv32.push_back((float)t.value); }
   m->dT = upload(c, m->T);
   m->dV = upload(c, m->V);
-  m->dTv64 = upload(c, tv64);
-  m->dTv32 = upload(c, tv32);
   m->dVv64 = upload(c, vv64);
   m->dVv32 = upload(c, vv32);
   split_interaction(m);
@@ -268,10 +265,12 @@ SpinCsr *get_spin(edgpu_model *m, int spin, int k) {
     launch_spin_ell(s->rp.as<int>(), s->col.as<int>(), s->v64.as<double>(), s->v32.as<float>(), (int)rows, s->ld,
                     s->len.as<int>(), s->ell_col.as<int>(), s->ell_v64.as<double>(), s->ell_v32.as<float>(), c->stream);
   }
-  s->uh64 = DBuf(c->alloc, sizeof(Hop<double>) * (size_t)std::max<long long>(1, s->nnz));
-  s->uh32 = DBuf(c->alloc, sizeof(Hop<float>) * (size_t)std::max<long long>(1, s->nnz));
-  launch_pack_hops<double>(s->col.as<int>(), s->v64.as<double>(), s->nnz, s->uh64.as<Hop<double>>(), c->stream);
-  launch_pack_hops<float>(s->col.as<int>(), s->v32.as<float>(), s->nnz, s->uh32.as<Hop<float>>(), c->stream);
+  if (spin == 0) {
+    s->uh64 = DBuf(c->alloc, sizeof(Hop<double>) * (size_t)std::max<long long>(1, s->nnz));
+    s->uh32 = DBuf(c->alloc, sizeof(Hop<float>) * (size_t)std::max<long long>(1, s->nnz));
+    launch_pack_hops<double>(s->col.as<int>(), s->v64.as<double>(), s->nnz, s->uh64.as<Hop<double>>(), c->stream);
+    launch_pack_hops<float>(s->col.as<int>(), s->v32.as<float>(), s->nnz, s->uh32.as<Hop<float>>(), c->stream);
+  }
   if (spin == 1 && rows >= kSrsLongRow && rows < kSrsVeryLong) {
     const int cells = std::max(1, s->kmax) * s->ld;
     s->slot4 = DBuf(c->alloc, sizeof(unsigned short) * cells);
@@ -337,7 +336,7 @@ static size_t ensure_masks(edgpu_model *m) {
 }
 
 template <typename T>
-void fill_common(edgpu_model *m, const Sector &s, SectorOp<T> &op, const T *diag, const T *tval, const T *vval) {
+void fill_common(edgpu_model *m, const Sector &s, SectorOp<T> &op, const T *diag, const T *vval) {
   op.storage = s.storage;
   op.ns = m->ns;
   op.ip = m->ip;
@@ -351,11 +350,8 @@ void fill_common(edgpu_model *m, const Sector &s, SectorOp<T> &op, const T *diag
   op.dn_basis = m->dbasis.as<int>() + m->basis_off[s.ndn];
   op.ninv_up = m->dninv.as<int>() + ((size_t)s.nup << m->ns);
   op.ninv_dn = m->dninv.as<int>() + ((size_t)s.ndn << m->ns);
-  op.nT = (int)m->T.size();
   op.nV = (int)m->V.size();
-  op.T_ = m->dT.as<Transition>();
   op.V_ = m->dV.as<Transition>();
-  op.T_val = tval;
   op.V_val = vval;
   op.nW = 0;
   op.nM = 0;
@@ -379,20 +375,16 @@ void ensure_ff(edgpu_model *m, Sector *s) {
     dst = DBuf(c->alloc, sizeof(ffloat) * (size_t)std::max<long long>(n, 1));
     launch_convert<ffloat>(src.as<double>(), dst.as<ffloat>(), n, c->stream);
   };
-  if (!m->dTvff.p) {
-    conv(m->dTvff, m->dTv64, (long long)m->T.size());
-    conv(m->dVvff, m->dVv64, (long long)m->V.size());
-  }
+  if (!m->dVvff.p) conv(m->dVvff, m->dVv64, (long long)m->V.size());
   SpinCsr *up = get_spin(m, 0, s->nup), *dn = get_spin(m, 1, s->ndn);
-  for (SpinCsr *sp : {up, dn}) {
-    if (!sp->vff.p) conv(sp->vff, sp->v64, sp->nnz);  // the CSR values are adopted buffers: counts, not bytes
-    if (!sp->ell_vff.p) conv(sp->ell_vff, sp->ell_v64, (long long)std::max(1, sp->kmax) * sp->ld);
-    if (!sp->uhff.p) {
-      sp->uhff = DBuf(c->alloc, sizeof(Hop<ffloat>) * (size_t)std::max<long long>(1, sp->nnz));
-      launch_pack_hops<ffloat>(sp->col.as<int>(), sp->vff.as<ffloat>(), sp->nnz, sp->uhff.as<Hop<ffloat>>(), c->stream);
-    }
-    if (sp->lv64.p && !sp->lvff.p) conv(sp->lvff, sp->lv64, (long long)std::max(1, sp->kmax) * sp->ld);
+  if (!up->uhff.p) {
+    conv(up->vff, up->v64, up->nnz);  // the CSR values are adopted buffers: counts, not bytes
+    up->uhff = DBuf(c->alloc, sizeof(Hop<ffloat>) * (size_t)std::max<long long>(1, up->nnz));
+    launch_pack_hops<ffloat>(up->col.as<int>(), up->vff.as<ffloat>(), up->nnz, up->uhff.as<Hop<ffloat>>(), c->stream);
   }
+  if (!dn->ell_vff.p) conv(dn->ell_vff, dn->ell_v64, (long long)std::max(1, dn->kmax) * dn->ld);
+  for (SpinCsr *sp : {up, dn})
+    if (sp->lv64.p && !sp->lvff.p) conv(sp->lvff, sp->lv64, (long long)std::max(1, sp->kmax) * sp->ld);
   conv(s->diagff, s->diag64, s->dim);
   const SectorOp<double> &d = s->op64;
   SectorOp<ffloat> &o = s->opff;
@@ -408,10 +400,6 @@ void ensure_ff(edgpu_model *m, Sector *s) {
   o.up_rp = d.up_rp;
   o.up_col = d.up_col;
   o.up_val = up->vff.as<ffloat>();
-  o.dn_rp = d.dn_rp;
-  o.dn_col = d.dn_col;
-  o.dn_val = dn->vff.as<ffloat>();
-  o.dn_nnz = d.dn_nnz;
   o.dn_len = d.dn_len;
   o.dn_ell_col = d.dn_ell_col;
   o.dn_ell_val = dn->ell_vff.as<ffloat>();
@@ -432,11 +420,8 @@ void ensure_ff(edgpu_model *m, Sector *s) {
   o.dn_basis = d.dn_basis;
   o.ninv_up = d.ninv_up;
   o.ninv_dn = d.ninv_dn;
-  o.nT = d.nT;
   o.nV = d.nV;
-  o.T_ = d.T_;
   o.V_ = d.V_;
-  o.T_val = m->dTvff.as<ffloat>();
   o.V_val = m->dVvff.as<ffloat>();
   o.nM = 0;
   o.M_ = nullptr;
@@ -473,8 +458,8 @@ Sector *get_sector(edgpu_model *m, int storage, int nup, int ndn) {
                                            std::to_string((size_t)s->dim * nTV) + ", allocated " + std::to_string(m->max_size) + ".");
   s->diag64 = DBuf(c->alloc, sizeof(double) * s->dim);
   s->diag32 = DBuf(c->alloc, sizeof(float) * s->dim);
-  fill_common<double>(m, *s, s->op64, s->diag64.as<double>(), m->dTv64.as<double>(), m->dVv64.as<double>());
-  fill_common<float>(m, *s, s->op32, s->diag32.as<float>(), m->dTv32.as<float>(), m->dVv32.as<float>());
+  fill_common<double>(m, *s, s->op64, s->diag64.as<double>(), m->dVv64.as<double>());
+  fill_common<float>(m, *s, s->op32, s->diag32.as<float>(), m->dVv32.as<float>());
   launch_diag(m->dm, s->op64, s->diag64.as<double>(), s->diag32.as<float>(), c->stream);
   if (storage == kSRS) {
     SpinCsr *up = get_spin(m, 0, nup), *dn = get_spin(m, 1, ndn);
@@ -482,11 +467,6 @@ Sector *get_sector(edgpu_model *m, int storage, int nup, int ndn) {
     s->op64.up_col = s->op32.up_col = up->col.as<int>();
     s->op64.up_val = up->v64.as<double>();
     s->op32.up_val = up->v32.as<float>();
-    s->op64.dn_rp = s->op32.dn_rp = dn->rp.as<int>();
-    s->op64.dn_col = s->op32.dn_col = dn->col.as<int>();
-    s->op64.dn_val = dn->v64.as<double>();
-    s->op32.dn_val = dn->v32.as<float>();
-    s->op64.dn_nnz = s->op32.dn_nnz = (int)dn->nnz;
     s->op64.dn_len = s->op32.dn_len = dn->len.as<int>();
     s->op64.dn_ell_col = s->op32.dn_ell_col = dn->ell_col.as<int>();
     s->op64.dn_ell_val = dn->ell_v64.as<double>();

@@ -206,10 +206,7 @@ struct SectorOp {
   // spin-resolved Kronecker pieces (SpinResolvedStorage.h:622-638)
   const int *up_rp, *up_col;
   const T *up_val;
-  const int *dn_rp, *dn_col;
-  const T *dn_val;
-  int dn_nnz;         // non-zeros of the down-spin CSR
-  // the same down-spin matrix k-major ("ELL"): entry k of row d at [k * dn_ld + d], row lengths dn_len[d];
+  // the down-spin matrix k-major ("ELL"): entry k of row d at [k * dn_ld + d], row lengths dn_len[d];
   // dn_ld = dn_rows rounded up to 4, so 4 consecutive rows load as one 16-byte vector
   const int *dn_len, *dn_ell_col;
   const T *dn_ell_val;
@@ -230,11 +227,9 @@ struct SectorOp {
   // tables for state <-> index and matrix-free transitions
   const int *up_basis, *dn_basis;    // masks of the C(Ns,N) states
   const int *ninv_up, *ninv_dn;      // ninv rows for N_up, N_dn
-  int nT, nV;                        // SRS: nV = 0 where the product tables below hold the interaction
-  const Transition *T_;
+  int nV;                            // SRS: 0 where the product tables below hold the interaction
   const Transition *V_;
-  const T *T_val;                    // transition values in vector precision
-  const T *V_val;
+  const T *V_val;                    // interaction values in vector precision
   // SOCRS: every transition (T and V) as masks, values with the constant part of the sign
   int nM;
   const TransMask *M_;

@@ -99,7 +99,7 @@ struct SpinCsr {
   DBuf rp, col, v64, v32;
   int kmax = 0, ld = 0;           // longest row; rows rounded up to 4
   DBuf len, ell_col, ell_v64, ell_v32;  // k-major copy (SectorOp::dn_ell_*)
-  DBuf uh64, uh32, uhff;           // the CSR entries as (column, value) pairs
+  DBuf uh64, uh32, uhff;           // up spin: the CSR entries as (column, value) pairs
   DBuf slot1, lv64, lv32, lvff;    // k-major entries in the order of a two-pass sector (SectorOp::long_*)
   DBuf tlen1;
   DBuf slot4, slot2;               // tile slots of the k-major columns, four and two columns per lane (SectorOp::dn_slot)
@@ -157,10 +157,10 @@ struct edgpu_model {
   std::vector<double> t, U, xmu, hmag, J, epsk, vk, h0, Ut;
   double mu = 0;
   size_t max_dim = 0, max_size = 0;
-  edgpu::host::DBuf dTvff, dVvff;  // float-float transition values (ensure_ff)
+  edgpu::host::DBuf dVvff;  // float-float interaction values (ensure_ff)
   edgpu::host::DBuf dM;  // every transition as masks, and their values (SectorOp::M_, M_val; ensure_masks)
   edgpu::host::VProd vprod;
-  edgpu::host::DBuf dT, dV, dTv64, dTv32, dVv64, dVv32, dU, dxmu, dhmag, dJ, depsk, dh0, dUt, dbinom, dbasis, dninv;
+  edgpu::host::DBuf dT, dV, dVv64, dVv32, dU, dxmu, dhmag, dJ, depsk, dh0, dUt, dbinom, dbasis, dninv;
   std::vector<long long> basis_off;
   edgpu::DevModel dm{};
   std::map<std::pair<int, int>, std::unique_ptr<edgpu::host::SpinCsr>> spin;
