@@ -62,7 +62,7 @@ struct RowPart {
 // meets a down hop of a column, where testing every transition on every state cost 24 state tests with two rank lookups
 // per hit.  (Not inlined: models without such terms keep the registers.)
 template <typename T, int C, int S>
-__device__ __noinline__ RowPart<T, C> srs_vloc(const SectorOp<T> *opp, int u, int d0, const T *__restrict__ x, RowPart<T, C> a) {
+__device__ __noinline__ RowPart<T, C> srs_vloc(const SectorOp<T> *opp, int u, int d0, const T *x, RowPart<T, C> a) {
   const SectorOp<T> &op = *opp;
   constexpr int U = 4;  // entries in flight
   const int Nd = op.dn_rows, ne = op.nW ? ldg_t(op.vu_cnt + u) : 0;
@@ -84,7 +84,7 @@ __device__ __noinline__ RowPart<T, C> srs_vloc(const SectorOp<T> *opp, int u, in
     for (int q = 0; q < U; ++q)
 #pragma unroll
       for (int cc = 0; cc < C; ++cc)
-        xv[q][cc] = to[q][cc] >= 0 ? ldg_t(x + (long long)en[q].x * Nd + (to[q][cc] >> 1)) : T(0);
+        xv[q][cc] = to[q][cc] >= 0 ? x[(long long)en[q].x * Nd + (to[q][cc] >> 1)] : T(0);
 #pragma unroll
     for (int q = 0; q < U; ++q)
 #pragma unroll
@@ -110,7 +110,7 @@ __device__ __noinline__ RowPart<T, C> srs_vloc(const SectorOp<T> *opp, int u, in
 
 // The same for R rows u, u + 1, ... (nr of them real) of one column: the rows' chains of loads run side by side.
 template <typename T, int R>
-__device__ __noinline__ RowPart<T, R> srs_vloc_rows(const SectorOp<T> *opp, int u, int nr, int d, const T *__restrict__ x,
+__device__ __noinline__ RowPart<T, R> srs_vloc_rows(const SectorOp<T> *opp, int u, int nr, int d, const T *x,
                                                     RowPart<T, R> a) {
   const SectorOp<T> &op = *opp;
   constexpr int U = 2;
@@ -142,7 +142,7 @@ __device__ __noinline__ RowPart<T, R> srs_vloc_rows(const SectorOp<T> *opp, int 
     for (int q = 0; q < U; ++q)
 #pragma unroll
       for (int r = 0; r < R; ++r)
-        xv[q][r] = to[q][r] >= 0 ? ldg_t(x + (long long)en[q][r].x * op.dn_rows + (to[q][r] >> 1)) : T(0);
+        xv[q][r] = to[q][r] >= 0 ? x[(long long)en[q][r].x * op.dn_rows + (to[q][r] >> 1)] : T(0);
 #pragma unroll
     for (int q = 0; q < U; ++q)
 #pragma unroll
@@ -209,6 +209,11 @@ __device__ __forceinline__ void fetch_item(SrsItem<T> &d, const SectorOp<T> *opp
   d.vloc = op.nW != 0 || op.nV != 0;
   d.skip = srs_two_pass(op.up_rows, Nd);  // k_srs_long's
 }
+
+// A recurrence's operator starts before the kernel that writes its x has ended (launch_pdl), and the read-only path
+// (ldg_t) asks for data that nobody writes while the kernel lives: x and z are read by ordinary loads, tables and the
+// diagonal through the read-only path.  Tiles of other launches read x through it too (RO; 495-state rows 106 instead of
+// 111 us).
 
 // C consecutive vector elements (16 bytes: 4 FP32 or 2 FP64) in one load when `vec` is set (the caller
 // guarantees the alignment); a ragged end (n < C) is read element by element.
@@ -296,8 +301,8 @@ struct TileGeom {
 enum TileMode { kVec, kOdd, kOff };
 
 // Rows [0, nrows) of Nd elements from x into the interleaved layout; the interleaved slots past the last row are zero.
-template <typename T, int M>
-__device__ __forceinline__ void stage_interleaved(T *xs, const T *__restrict__ x, int nrows, int Nd) {
+template <typename T, int M, bool RO>
+__device__ __forceinline__ void stage_interleaved(T *xs, const T *x, int nrows, int Nd) {
   constexpr int RI = TileGeom<T>::RI, C = TileGeom<T>::C;
   const int nq = (nrows + RI - 1) / RI;
   Lanes<T> *out = reinterpret_cast<Lanes<T> *>(xs);
@@ -308,7 +313,7 @@ __device__ __forceinline__ void stage_interleaved(T *xs, const T *__restrict__ x
     for (int e = threadIdx.x; e < nq * Nq; e += kMvBlock) {
       Lanes<T> v[RI];
 #pragma unroll
-      for (int i = 0; i < RI; ++i) v[i] = q * RI + i < nrows ? ldg16(x + (q * RI + i) * Nd + C * d) : Lanes<T>{};
+      for (int i = 0; i < RI; ++i) v[i] = q * RI + i < nrows ? (RO ? ldg16(x + (q * RI + i) * Nd + C * d) : load16(x + (q * RI + i) * Nd + C * d)) : Lanes<T>{};
 #pragma unroll
       for (int cc = 0; cc < C; ++cc) {
         Lanes<T> w;
@@ -325,7 +330,7 @@ __device__ __forceinline__ void stage_interleaved(T *xs, const T *__restrict__ x
     for (int e = threadIdx.x; e < nq * Nd; e += kMvBlock) {
       Lanes<T> v;
 #pragma unroll
-      for (int i = 0; i < RI; ++i) v.v[i] = q * RI + i < nrows ? ldg_t(x + (q * RI + i) * Nd + d) : T(0);
+      for (int i = 0; i < RI; ++i) v.v[i] = q * RI + i < nrows ? (RO ? ldg_t(x + (q * RI + i) * Nd + d) : x[(q * RI + i) * Nd + d]) : T(0);
       out[q * Nd + (M == kOdd ? d : tile_slot(d, Nd, C))] = v;
       q += qs;
       d += ds;
@@ -371,7 +376,7 @@ struct ItemHops {
 // Per element the sum runs diagonal, (c z), down hops and up hops each in the reference's order, interaction: another
 // order (down hops dealt out so that a phase's eight lanes meet few bank conflicts) is faster, but the eigen-solver's
 // and the recurrences' vectors are then others in the last bit, which unconverged quantities magnify.
-template <typename T, int M, int HB, bool MZ, bool MD>
+template <typename T, int M, int HB, bool MZ, bool MD, bool RO>
 __device__ __forceinline__ void srs_tile(const SrsItem<T> &it, const ItemHops<T> &hops, int rg, int cb, int c0, bool mine,
                                          const T *__restrict__ xs, DotAcc &acc) {
   using TG = TileGeom<T>;
@@ -458,7 +463,7 @@ __device__ __forceinline__ void srs_tile(const SrsItem<T> &it, const ItemHops<T>
       nmax = max(nmax, n[r]);
     }
     if (!mine) nmax = 0;
-    const T *__restrict__ xc = it.x + c0;
+    const T *xc = it.x + c0;
 #pragma unroll 1
     for (int h = 0; h < nmax; h += HB) {
       T xq[R][HB][C], v[R][HB];
@@ -468,7 +473,7 @@ __device__ __forceinline__ void srs_tile(const SrsItem<T> &it, const ItemHops<T>
         for (int q = 0; q < HB; ++q) {
           const Hop<T> hp = hops.hop[h + q < n[r] ? k0[r] + h + q : none];
           v[r][q] = hp.v;
-          ld_tile<T, C, VEC>(xc + hp.c, o, xq[r][q]);
+          ld_tile<T, C, VEC, RO>(xc + hp.c, o, xq[r][q]);
         }
 #pragma unroll
       for (int r = 0; r < R; ++r)
@@ -514,7 +519,7 @@ __device__ __forceinline__ void srs_tile(const SrsItem<T> &it, const ItemHops<T>
 // 8-byte types, bound by arithmetic, whose cost does not fall with idle lanes, and for rows that leave more than a
 // ninth of the tiles' columns empty (FP32 rows of 220 states).  With dot products (MD) a thread's elements are part of
 // the sums' values: kVec units numbered through, other tiles not moved.
-template <typename T, int M, int HB, bool MZ, bool MD>
+template <typename T, int M, int HB, bool MZ, bool MD, bool RO>
 __device__ __forceinline__ DotAcc srs_tiles(const SrsItem<T> &it, const ItemHops<T> &hops, const T *__restrict__ xs) {
   using TG = TileGeom<T>;
   constexpr int C = TG::C;
@@ -527,15 +532,15 @@ __device__ __forceinline__ DotAcc srs_tiles(const SrsItem<T> &it, const ItemHops
   for (int unit = linear ? threadIdx.x : threadIdx.x >> 5; unit < ngr * per; unit += linear ? kMvBlock : kMvBlock / 32) {
     const int g = unit / per, q = unit - g * per;
     const int cb = linear ? 0 : q * TG::W, want = linear ? q * C : M == kVec ? cb + C * lane : (MD ? cb : min(cb, it.Nd - TG::W)) + lane;
-    srs_tile<T, M, HB, MZ, MD>(it, hops, g * TG::R, cb, M == kVec ? min(want, it.Nd - C) : want, want < it.Nd,
+    srs_tile<T, M, HB, MZ, MD, RO>(it, hops, g * TG::R, cb, M == kVec ? min(want, it.Nd - C) : want, want < it.Nd,
                                xs, acc);
   }
   return acc;
 }
 // tiles off 16-byte bases apart from the others, with registers of their own
-template <typename T, bool MZ, bool MD>
+template <typename T, bool MZ, bool MD, bool RO>
 __device__ __noinline__ DotAcc srs_tiles_off(const SrsItem<T> &it, const ItemHops<T> &hops, const T *__restrict__ xs) {
-  return srs_tiles<T, kOff, 1, MZ, MD>(it, hops, xs);
+  return srs_tiles<T, kOff, 1, MZ, MD, RO>(it, hops, xs);
 }
 
 // SRS item of very long rows (one to three rows per item, each staged in shared memory): one row at a time,
@@ -549,9 +554,8 @@ constexpr int kLongHops = 128;
 template <typename T, bool MZ, bool MD>
 __device__ __noinline__ DotAcc srs_longrow(const SrsItem<T> &it, const T *__restrict__ xs) {
   const SectorOp<T> &op = *it.op;
-  const T *__restrict__ x = it.x;
-  const T *z = it.z;
-  T *__restrict__ y = it.y;
+  const T *x = it.x, *z = it.z;
+  T *y = it.y;
   const T c = it.c;
   const int u0 = it.u0, nrows = it.nrows;
   DotAcc acc;
@@ -607,12 +611,11 @@ __device__ __noinline__ DotAcc srs_longrow(const SrsItem<T> &it, const T *__rest
             const int hq = h + q < nh ? h + q : h;
             const T *src = x + hop_off[hq] + d0;
             if constexpr (sizeof(T) == 4) {
-              const float2 p0 = ldg_t(reinterpret_cast<const float2 *>(src));
-              const float2 p1 = ldg_t(reinterpret_cast<const float2 *>(src + 2));
+              const float2 p0 = *reinterpret_cast<const float2 *>(src), p1 = *reinterpret_cast<const float2 *>(src + 2);
               xq[q].v[0] = p0.x, xq[q].v[1] = p0.y, xq[q].v[2] = p1.x, xq[q].v[3] = p1.y;
             } else {
-              xq[q].v[0] = ldg_t(src);
-              xq[q].v[1] = ldg_t(src + 1);
+              xq[q].v[0] = src[0];
+              xq[q].v[1] = src[1];
             }
           }
 #pragma unroll
@@ -629,7 +632,7 @@ __device__ __noinline__ DotAcc srs_longrow(const SrsItem<T> &it, const T *__rest
           const T *src = x + hop_off[h] + d0;
 #pragma unroll
           for (int cc = 0; cc < C; ++cc)
-            if (cc < nc) a[cc] += v * ldg_t(src + cc);
+            if (cc < nc) a[cc] += v * src[cc];
         }
       }
       for (int h = nh; h < nall; ++h) {
@@ -637,7 +640,7 @@ __device__ __noinline__ DotAcc srs_longrow(const SrsItem<T> &it, const T *__rest
         const T *src = x + (long long)ldg_t(op.up_col + k0 + h) * Nd + d0;
 #pragma unroll
         for (int cc = 0; cc < C; ++cc)
-          if (cc < nc) a[cc] += v * ldg_t(src + cc);
+          if (cc < nc) a[cc] += v * src[cc];
       }
       if (op.nW != 0 || op.nV != 0) {
         RowPart<T, C> p;
@@ -704,7 +707,7 @@ __device__ __noinline__ void srs_short(const SrsItem<T> &it, const ItemHops<T> &
       nh[r] = ldg_t(p + 1) - k0[r];
       nmax = max(nmax, nh[r]);
     }
-    const T *__restrict__ xd = it.x + d;
+    const T *xd = it.x + d;
     const int first = ldg_t(it.urp);
 #pragma unroll 1
     for (int h = 0; h < nmax; h += 4) {
@@ -723,7 +726,7 @@ __device__ __noinline__ void srs_short(const SrsItem<T> &it, const ItemHops<T> &
               hp.c *= Nd;
             }
             v[q][r] = hp.v;
-            xq[q][r] = ldg_t(xd + hp.c);
+            xq[q][r] = xd[hp.c];
           }
         }
 #pragma unroll
@@ -773,7 +776,7 @@ __device__ __noinline__ DotAcc srs_flat(const SrsItem<T> &it, const ItemHops<T> 
 #pragma unroll 4
     for (int k = 0; k < kk; ++k) a = madd(ldg_t(eval + k * ld + d), xg[ldg_t(ecol + k * ld + d) * RI], a);
     const int k0 = ldg_t(it.urp + r), nh = ldg_t(it.urp + r + 1) - k0;
-    const T *__restrict__ xd = it.x + d;
+    const T *xd = it.x + d;
 #pragma unroll 4
     for (int h = 0; h < nh; ++h) {
       Hop<T> hp;
@@ -783,7 +786,7 @@ __device__ __noinline__ DotAcc srs_flat(const SrsItem<T> &it, const ItemHops<T> 
         hp = ldg_hop(it.uh + k0 + h);
         hp.c *= Nd;
       }
-      a = madd(hp.v, ldg_t(xd + hp.c), a);
+      a = madd(hp.v, xd[hp.c], a);
     }
     if (it.vloc) a = srs_vloc<T, 1, 1>(it.op, it.u0 + r, d, it.x, RowPart<T, 1>{{a}}).v[0];
     it.y[e] = renorm(a);
@@ -802,8 +805,7 @@ __device__ __noinline__ DotAcc srs_flat(const SrsItem<T> &it, const ItemHops<T> 
 // their loads in flight; in FP64 one lane per row also keeps a warp's additions to one per transition, where eight lanes
 // per row (butterfly, or handed around in order) took eight times the FP64 issue slots.
 template <typename T, int ST>
-__device__ __forceinline__ void mv_item(const SectorOp<T> *opp, int rows, long long li, const T *__restrict__ x,
-                                        T *__restrict__ y, const T *z, T c) {
+__device__ __forceinline__ void mv_item(const SectorOp<T> *opp, int rows, long long li, const T *x, T *y, const T *z, T c) {
   const SectorOp<T> &op = *opp;
   constexpr int U = 4;
   long long lo, hi;
@@ -954,6 +956,7 @@ struct EigSource {
 // at compile time); HB: up hops in flight per row of a tile; MB: resident blocks per SM its registers are held to.
 template <typename T, class Src, bool MZ, bool MD, int HB, int MB>
 __global__ void __launch_bounds__(kMvBlock, MB) k_srs_mv(Src src, int nitems, int xs_cap, int hop_cap) {
+  constexpr bool RO = !Src::kEarly;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ SrsItem<T> items[2];
   __shared__ double red[kMvBlock / 32];
@@ -1002,11 +1005,11 @@ __global__ void __launch_bounds__(kMvBlock, MB) k_srs_mv(Src src, int nitems, in
         }
     }
     if (tile) {
-      if (vec) stage_interleaved<T, kVec>(xs, it.xi, it.nrows, Nd);
-      else if (!whole) stage_interleaved<T, kOdd>(xs, it.xi, it.nrows, Nd);
-      else stage_interleaved<T, kOff>(xs, it.xi, it.nrows, Nd);
+      if (vec) stage_interleaved<T, kVec, RO>(xs, it.xi, it.nrows, Nd);
+      else if (!whole) stage_interleaved<T, kOdd, RO>(xs, it.xi, it.nrows, Nd);
+      else stage_interleaved<T, kOff, RO>(xs, it.xi, it.nrows, Nd);
     } else if (small) {
-      stage_interleaved<T, kOdd>(xs, it.xi, it.nrows, Nd);
+      stage_interleaved<T, kOdd, RO>(xs, it.xi, it.nrows, Nd);
     } else if (nel <= xs_cap) {
       stage_async(xs, it.xi, nel);
     }
@@ -1015,9 +1018,9 @@ __global__ void __launch_bounds__(kMvBlock, MB) k_srs_mv(Src src, int nitems, in
     __syncthreads();
     DotAcc acc{};
     if (tile) {
-      if (vec) acc = srs_tiles<T, kVec, HB, MZ, MD>(it, hops, xs);
-      else if (!whole) acc = srs_tiles<T, kOdd, HB, MZ, MD>(it, hops, xs);
-      else acc = srs_tiles_off<T, MZ, MD>(it, hops, xs);
+      if (vec) acc = srs_tiles<T, kVec, HB, MZ, MD, RO>(it, hops, xs);
+      else if (!whole) acc = srs_tiles<T, kOdd, HB, MZ, MD, RO>(it, hops, xs);
+      else acc = srs_tiles_off<T, MZ, MD, RO>(it, hops, xs);
     } else if (small) {
       if constexpr (MD) acc = srs_flat<T, MZ>(it, hops, near, xs);
       else srs_short<T, MZ>(it, hops, near, xs);
