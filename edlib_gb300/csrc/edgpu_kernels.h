@@ -136,11 +136,14 @@ __host__ __device__ inline bool srs_two_pass(int up_rows, int dn_rows) {
 // shared memory; rows longer than 6144 elements one or a few per item); short rows take about kItemElems
 // elements per item.  Measured on Anderson-12 (FP32 eigen-solve of all sectors): 0.575 s with 4096, 0.531 s
 // with 8192, 0.543 s with 16384, 0.595 s with 2048 elements per item.
+// most elements of a tiled item: with 8-byte ones 96 KB, which leaves room for the item's up hops (up to 64 rows of 100,
+// 16 bytes each, when every site of 20 is bound to every other) in the 227 KB of a block
+constexpr int kTileElems = 12288;
 inline int srs_item_elems() {
   static const int target = [] {  // elements per item of long rows (EDGPU_SRS_ITEM_ELEMS, for measurements)
     const char *e = getenv("EDGPU_SRS_ITEM_ELEMS");
     const int v = e ? atoi(e) : 0;
-    return v >= 512 && v <= 24576 ? v : 8192;  // 8192: 8 % less eigen-solve time than 4096 on Anderson-12
+    return v >= 512 && v <= 24576 ? std::min(v, kTileElems) : 8192;
   }();
   return target;
 }
@@ -148,7 +151,7 @@ inline int srs_item_rows(int up_rows, int dn_rows) {
   if (srs_two_pass(up_rows, dn_rows)) return kLongRows;
   const int target = srs_item_elems();
   int r;
-  if (dn_rows >= kSrsLongRow && dn_rows < kSrsVeryLong) r = std::max(4, std::min(24576 / dn_rows, target / dn_rows) & ~3);
+  if (dn_rows >= kSrsLongRow && dn_rows < kSrsVeryLong) r = std::max(4, target / dn_rows & ~3);
   else if (dn_rows >= kSrsLongRow) r = std::max(1, 24576 / dn_rows);  // very long rows: as many as stage in 96 KB
   else r = kItemElems / std::max(1, dn_rows);
   // small sectors of short rows, which leave SMs idle: 512 elements or four rows
@@ -165,7 +168,7 @@ inline int lz_item_rows(int storage, int up_rows, int dn_rows) {
   if (storage != kSRS) return kItemElems;
   if (dn_rows >= kSrsVeryLong) return srs_item_rows(up_rows, dn_rows);
   const int r = dn_rows < kSrsLongRow ? kItemElems / std::max(1, dn_rows)
-                                      : std::min(kTileRows, std::max(4, std::min(24576, srs_item_elems()) / dn_rows & ~3));
+                                      : std::min(kTileRows, std::max(4, srs_item_elems() / dn_rows & ~3));
   return std::max(1, std::min(r, up_rows));
 }
 

@@ -245,3 +245,40 @@ def test_items_across_the_sectors_own_ones(ed, precision, ns, sec, nvec):
     w = o.av(x[0, :n].double().cpu().numpy())
     assert np.abs(ys[0][0].double().cpu().numpy() - w).max() <= TOL[precision] * np.abs(w).max()
     ham.close()
+
+
+# item sizes at both ends of EDGPU_SRS_ITEM_ELEMS (read once, so in a fresh process), on a cluster whose sites are all bound
+# to one another: most up hops per item
+@pytest.mark.parametrize("elems", [512, 24576])
+def test_item_sizes_against_oracle(elems):
+    import os
+    import subprocess
+    import sys
+    code = (
+        "import numpy as np\n"
+        "from edlib_gb300 import ed, models\n"
+        "from oracle.oracle import OracleED\n"
+        "ed.context(0)\n"
+        "rng = np.random.default_rng(9)\n"
+        "t = rng.uniform(0.2, 1.0, (14, 14))\n"
+        "t = t + t.T - np.diag(np.diag(t + t.T))\n"
+        "params = {'NSITES': 14, 'NSPINS': 2, 'storage.MAX_DIM': 0, 'storage.MAX_SIZE': 0}\n"
+        "data = models.hubbard(t, 3.0, 1.0)\n"
+        "ham = ed.Hamiltonian(params, data, storage='SRS', precision='fp64')\n"
+        "ham.set_limits(0, 0)\n"
+        "o = OracleED(params, data, 'SRS', 'HUBBARD')\n"
+        "for sec in [(7, 3), (6, 11)]:\n"
+        "    n = ham.storage.fill(*sec)\n"
+        "    assert o.fill(*sec) == n\n"
+        "    v = rng.standard_normal(n)\n"
+        "    w = o.av(v)\n"
+        "    assert np.abs(ham.storage.av(v) - w).max() <= 1e-13 * np.abs(w).max(), sec\n"
+        "    v /= np.linalg.norm(v)\n"
+        "    a, b, _ = ed.lanczos(ham, sec, v, 3)\n"
+        "    w = o.av(v)\n"
+        "    assert abs(a[0, 0] - w @ v) <= 1e-12 and abs(b[0, 1] - np.linalg.norm(w - (w @ v) * v)) <= 1e-12, sec\n"
+        "print('ok')\n")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=900,
+                       env=dict(os.environ, EDGPU_SRS_ITEM_ELEMS=str(elems), PYTHONPATH=root))
+    assert r.returncode == 0 and "ok" in r.stdout, r.stderr[-3000:]
