@@ -116,9 +116,10 @@ void launch_diag(const DevModel &m, const SectorOp<double> &op, double *d64, flo
 void launch_socrs_check(const DevModel &m, const SectorOp<double> &op, int *err, cudaStream_t st);
 
 // ---- spmv.cuh / krylov.cu : batched operator kernels
-// Element range of item li of a sector operator.
-// SRS sectors whose rows (down-spin dimension) are at least this long are swept by thread-per-column
-// tiles of several rows; shorter rows are spread flat over the block.
+// SMs of a GB300: item sizes aim at one or two items per SM where a sector is small.
+constexpr int kSms = 152;
+// SRS sectors whose rows (down-spin dimension) are at least this long are swept in tiles of four rows; of shorter rows a
+// thread takes one column of a few rows at a time (spmv.cuh: srs_tile, srs_short).
 constexpr int kSrsLongRow = 128;
 constexpr int kSrsVeryLong = 4096;  // rows from here on do not go four at a time into a tile's shared memory
 constexpr int kTileRows = 64;       // most up-spin rows of a tiled item (kSrsLongRow <= row < kSrsVeryLong)
@@ -131,11 +132,12 @@ constexpr int kLongUp = 512, kLongMax = 224 * 1024 / 16, kLongRows = 4;
 __host__ __device__ inline bool srs_two_pass(int up_rows, int dn_rows) {
   return dn_rows >= kSrsVeryLong && dn_rows <= kLongMax && up_rows >= kLongUp && up_rows <= kLongMax;
 }
-// Up-spin rows per SRS work item: long rows are swept in groups of 4 rows, about 8192 elements per item
-// (EDGPU_SRS_ITEM_ELEMS; at most 24576, as many rows as fit 96 KB of FP32, so that they still stage in
-// shared memory; rows longer than 6144 elements one or a few per item); short rows take about kItemElems
-// elements per item.  Measured on Anderson-12 (FP32 eigen-solve of all sectors): 0.575 s with 4096, 0.531 s
-// with 8192, 0.543 s with 16384, 0.595 s with 2048 elements per item.
+// Up-spin rows per SRS work item.  Rows of kSrsLongRow to kSrsVeryLong - 1 states go in groups of four, 8192 elements per
+// item (EDGPU_SRS_ITEM_ELEMS: 512 to 24576, cut to kTileElems), but no fewer items than one per SM where that leaves four
+// rows each; longer rows one to three per item (or kLongRows in two passes); of shorter ones about kItemElems elements, in
+// sectors that would leave SMs idle 512.  The size of tiled items hardly matters for the batch of all sectors of the
+// 12-orbital impurity (its solve 283 ms with 2048 elements, 278 with 4096, 279 with 6144, 281 with 8192, 289 with 12288),
+// more for single large sectors (their recurrences 27.9, 27.9, 27.9, 26.2, 30.5 ms).
 // most elements of a tiled item: with 8-byte ones 96 KB, which leaves room for the item's up hops (up to 64 rows of 100,
 // 16 bytes each, when every site of 20 is bound to every other) in the 227 KB of a block
 constexpr int kTileElems = 12288;
@@ -158,7 +160,7 @@ inline int srs_item_rows(int up_rows, int dn_rows) {
   if (dn_rows < kSrsLongRow && (long long)up_rows * dn_rows <= 8192) r = std::min(r, std::max(4, 512 / dn_rows & ~3));
   // sectors of too few rows for an item per SM of that size: about one item per SM, of at least four rows
   if (dn_rows >= kSrsLongRow && dn_rows < kSrsVeryLong)
-    r = std::min({r, kTileRows, std::max(4, ((up_rows + 151) / 152 + 3) & ~3)});
+    r = std::min({r, kTileRows, std::max(4, ((up_rows + kSms - 1) / kSms + 3) & ~3)});
   return std::max(1, std::min(r, up_rows));
 }
 
@@ -175,8 +177,8 @@ inline int lz_item_rows(int storage, int up_rows, int dn_rows) {
 // SRS rows per item of a product of nvec vectors of one sector (edgpu_spmv): the sector's own, or, where those make too few
 // items for two per SM, as few as that takes, in groups of four.
 inline int vec_item_rows(int srs_rows, int up_rows, int dn_rows, int nitems, long long nvec) {
-  if (dn_rows >= kSrsVeryLong || nvec * nitems >= 304) return srs_rows;
-  return (int)std::min<long long>(srs_rows, std::max<long long>(4, (nvec * up_rows / 304 + 3) / 4 * 4));
+  if (dn_rows >= kSrsVeryLong || nvec * nitems >= 2 * kSms) return srs_rows;
+  return (int)std::min<long long>(srs_rows, std::max<long long>(4, (nvec * up_rows / (2 * kSms) + 3) / 4 * 4));
 }
 
 // Room in shared memory for the up hops of an item (entries): of any srs_rows consecutive rows, from the longest row,
@@ -189,10 +191,10 @@ inline int item_hop_room(int srs_rows, int dn_rows, int kmax) {
   return dn_rows < kSrsLongRow ? std::min(n, 1024) : n;
 }
 
-// Rows per item of a CRS or SOCRS sector: about two items per SM, of 64 to 2048 rows (4900 rows in items of 2048
+// Rows per item of a CRS or SOCRS product: about two items per SM, of 64 to 2048 rows (4900 rows in items of 2048
 // left all but three SMs idle).
 inline int row_item(long long dim) {
-  return (int)std::min<long long>(kItemElems, std::max<long long>(64, (dim / 304 + 63) / 64 * 64));
+  return (int)std::min<long long>(kItemElems, std::max<long long>(64, (dim / (2 * kSms) + 63) / 64 * 64));
 }
 template <typename T>
 __host__ __device__ inline void item_range(const SectorOp<T> &op, int srs_rows, long long li, long long &lo, long long &hi) {
