@@ -275,10 +275,9 @@ int edgpu_spmv(edgpu_model *m, int storage, int nup, int ndn, const void *x, voi
       Sector_mv<T> v{s->dop<T>(), static_cast<const T *>(x), static_cast<T *>(y), ldx, nvec, s->srs_rows, s->nitems,
                      accumulate != 0};
       MvShape sh = mv_shape<T>(*s);
-      if (s->storage == kSRS) {
-        v.rows = vec_item_rows(s->srs_rows, s->up_rows, s->dn_rows, s->nitems, nvec);
-        v.per = (s->up_rows + v.rows - 1) / v.rows;
-      }
+      v.rows = s->storage == kSRS ? vec_item_rows(s->srs_rows, s->up_rows, s->dn_rows, s->nitems, nvec)
+                                  : row_item(s->dim * nvec, 64);
+      v.per = (int)(((s->storage == kSRS ? s->up_rows : s->dim) + v.rows - 1) / v.rows);
       if ((long long)v.per * nvec > INT_MAX) throw ApiError(EDGPU_ERR_ARG, "too many vectors for one call");
       launch_mv_vectors<T>(v, sh, st);
       CK(cudaGetLastError());

@@ -500,7 +500,7 @@ Sector *get_sector(edgpu_model *m, int storage, int nup, int ndn) {
     s->nitems = (s->up_rows + s->srs_rows - 1) / s->srs_rows;
     s->up_kmax = up->kmax;
   } else {
-    s->srs_rows = row_item(s->dim);
+    s->srs_rows = row_item(s->dim, 128);  // an eigen-solver step has many sectors
     s->nitems = (int)((s->dim + s->srs_rows - 1) / s->srs_rows);
   }
   s->lz_rows = lz_item_rows(storage, s->up_rows, s->dn_rows);

@@ -191,10 +191,12 @@ inline int item_hop_room(int srs_rows, int dn_rows, int kmax) {
   return dn_rows < kSrsLongRow ? std::min(n, 1024) : n;
 }
 
-// Rows per item of a CRS or SOCRS product: about two items per SM, of 64 to 2048 rows (4900 rows in items of 2048
-// left all but three SMs idle).
-inline int row_item(long long dim) {
-  return (int)std::min<long long>(kItemElems, std::max<long long>(64, (dim / (2 * kSms) + 63) / 64 * 64));
+// Rows per item of CRS or SOCRS products over `rows` rows in all: about three items per SM, of `least` to 256 rows, one per
+// thread (4900 rows in items of 2048 left all but three SMs idle; 48 vectors of them in items of 64 left three quarters of
+// each block's threads idle, 43 instead of 32 us; 15 vectors of 63,504 rows in items of 2048 make one wave with a tail,
+// 37 instead of 31 us).
+inline int row_item(long long rows, int least) {
+  return (int)std::min<long long>(256, std::max<long long>(least, (rows / (3 * kSms) + 63) / 64 * 64));
 }
 template <typename T>
 __host__ __device__ inline void item_range(const SectorOp<T> &op, int srs_rows, long long li, long long &lo, long long &hi) {

@@ -798,42 +798,35 @@ __device__ __noinline__ DotAcc srs_flat(const SrsItem<T> &it, const ItemHops<T> 
   return acc;
 }
 
-// One item of a sector: y[lo:hi) = (H x)[lo:hi) + c z[lo:hi), every row added in its own order.  CRS: four lanes share a
-// row; they read its entries side by side, U rounds of them in flight, and each adds all of them, handed around by
-// shuffles.  (One thread per row waited for its own chain of loads: 4900 rows of 17 entries, one FP64 vector, 27 us cold
-// in three items of 2048 rows.)  SOCRS: a thread per row tests the transitions by their masks (TransMask), U of them with
-// their loads in flight; in FP64 one lane per row also keeps a warp's additions to one per transition, where eight lanes
-// per row (butterfly, or handed around in order) took eight times the FP64 issue slots.
+// One item of a sector: y[lo:hi) = (H x)[lo:hi) + c z[lo:hi), a thread per row, the row added in its own order, U of its
+// entries (CRS) or transitions (SOCRS, tested by their masks: TransMask) with their loads in flight.  Items are small
+// enough for every SM (row_item): 4900 rows of 17 entries, one FP64 vector, 27 us cold in three items of 2048 rows.
+// Several lanes per row, reading its entries side by side, add by a butterfly (another sum) or hand all entries around,
+// and then every lane adds all of them: FP64 issue, two lanes per clock and SM, bounds that (63,504 CRS rows, 15 FP64
+// vectors: 129 us with four lanes per row).
 template <typename T, int ST>
 __device__ __forceinline__ void mv_item(const SectorOp<T> *opp, int rows, long long li, const T *x, T *y, const T *z, T c) {
   const SectorOp<T> &op = *opp;
-  constexpr int U = 4;
+  constexpr int U = ST == kCRS ? 4 : 4;
   long long lo, hi;
   item_range(op, rows, li, lo, hi);
   if constexpr (ST == kCRS) {
-    constexpr int L = 4;
-    const int q = threadIdx.x % L;
-    const unsigned group = ((1u << L) - 1) << ((threadIdx.x & 31) - q);
-    for (long long i = lo + threadIdx.x / L; i < hi; i += kMvBlock / L) {  // a row's lanes stay together
+    for (long long i = lo + threadIdx.x; i < hi; i += kMvBlock) {
       const long long j1 = op.crs_rp[i + 1];
       T v = z ? mul_rn(c, z[i]) : T(0);
-      for (long long j = op.crs_rp[i] + q; j - q < j1; j += U * L) {
+      for (long long j = op.crs_rp[i]; j < j1; j += U) {
         T a[U], b[U];
 #pragma unroll
         for (int k = 0; k < U; ++k) {
-          const bool in = j + k * L < j1;
-          a[k] = in ? ldg_t(op.crs_val + j + k * L) : T(0);
-          b[k] = in ? x[__ldg(op.crs_col + j + k * L)] : T(0);
+          const bool in = j + k < j1;
+          a[k] = in ? ldg_t(op.crs_val + j + k) : T(0);
+          b[k] = in ? x[__ldg(op.crs_col + j + k)] : T(0);
         }
 #pragma unroll
         for (int k = 0; k < U; ++k)
-#pragma unroll
-          for (int p = 0; p < L; ++p) {
-            const T av = __shfl_sync(group, a[k], p, L), bv = __shfl_sync(group, b[k], p, L);
-            if (j - q + k * L + p < j1) v = madd(av, bv, v);
-          }
+          if (j + k < j1) v = madd(a[k], b[k], v);
       }
-      if (q == 0) y[i] = v;
+      y[i] = v;
     }
   } else {
     const unsigned Nd = (unsigned)op.dn_rows;
