@@ -986,7 +986,9 @@ __global__ void __launch_bounds__(kMvBlock, MB) k_srs_mv(Src src, int nitems, in
     if (tile || small) {
       const int k0 = ldg_t(it.urp), nh = ldg_t(it.urp + it.nrows) - k0;
       near = nh <= hop_cap;
-      tile = tile && near;  // else row by row from global memory
+      // else row by row from global memory; so are a recurrence's last rows of 2048 states or more, fewer than a group of
+      // four, whose <x, y> is summed in that order
+      tile = tile && near && !(MD && it.dot && it.nrows < TileGeom<T>::R && Nd >= 2048);
       if (tile)
         for (int q = threadIdx.x; q <= it.nrows; q += kMvBlock) hop_rp[q] = ldg_t(it.urp + q) - k0;
       if (near)
