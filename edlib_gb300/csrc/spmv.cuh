@@ -364,8 +364,8 @@ struct ItemHops {
 };
 
 // A thread's part of a tile of the SRS sweep: rows rg .. rg + 3 of the item (those below nrows), columns from c0 on
-// (kVec: C consecutive ones; else 32 apart).  Columns below cb are another tile's, columns past the row's end (MD) and the
-// lanes that are not `mine` repeat others, and so do rows past the item's end; all of them store nothing: every load is
+// (kVec: C consecutive ones; else 32 apart).  Columns below cb are another tile's, columns past the row's end (MD; `mine`
+// says whether c0 is one) repeat the last, and so do rows past the item's end; all of them store nothing: every load is
 // in bounds without a predicate.
 // What bounds it: L1 and shared-memory wavefronts, then issue slots.  Rows apart in shared memory (each down-hop
 // entry 16 address computations and 16 scalar loads per thread) took 110 thread instructions per state.  Here an
@@ -387,7 +387,7 @@ __device__ __forceinline__ void srs_tile(const SrsItem<T> &it, const ItemHops<T>
   int o[C];  // the columns, from c0
 #pragma unroll
   for (int cc = 0; cc < C; ++cc) o[cc] = VEC ? cc : MD ? min(32 * cc, Nd - 1 - c0) : 32 * cc;
-  auto own = [&](int cc) { return VEC ? mine : MD ? c0 + 32 * cc < Nd : c0 + 32 * cc >= cb; };
+  auto own = [&](int cc) { return VEC ? true : MD ? c0 + 32 * cc < Nd : c0 + 32 * cc >= cb; };
   auto slot = [&](int cc) { return VEC ? c0 / C + cc * (Nd / C) : M == kOdd ? c0 + o[cc] : tile_slot(c0 + o[cc], Nd, C); };
   auto row = [&](int r) { return min(rg + r, it.nrows - 1) * Nd + c0; };
   T a[R][C];
@@ -498,7 +498,7 @@ __device__ __forceinline__ void srs_tile(const SrsItem<T> &it, const ItemHops<T>
     }
     T *__restrict__ y = it.y + row(r);
     if constexpr (VEC) {
-      if (mine) store_lanes(y, a[r]);
+      store_lanes(y, a[r]);
     } else {
 #pragma unroll
       for (int cc = 0; cc < C; ++cc)
@@ -512,28 +512,25 @@ __device__ __forceinline__ void srs_tile(const SrsItem<T> &it, const ItemHops<T>
   }
 }
 
-// The tiles of a staged item; the thread's part of <x, y>.  Either a warp per tile of 4 rows x W columns, so that a
-// shared-memory phase's eight lanes hold neighbouring columns; past the row's end kVec lanes take
-// the last columns again (the same addresses as their owner's, no extra wavefront), the others' tiles move back to
-// end with the row.  Or the units of a kVec item numbered through, a thread each, rows ending inside a warp: for
-// 8-byte types, bound by arithmetic, whose cost does not fall with idle lanes, and for rows that leave more than a
-// ninth of the tiles' columns empty (FP32 rows of 220 states).  With dot products (MD) a thread's elements are part of
-// the sums' values: kVec units numbered through, other tiles not moved.
+// The tiles of a staged item; the thread's part of <x, y>.  kVec: the item's units of 4 rows x C columns numbered through, a
+// thread each, rows ending inside a warp.  (A warp per tile of 4 rows x W columns, the last columns taken twice past the
+// row's end, is 1 % faster on FP32 rows of 220 or 560 states, the same on 252, 792, 816, 924 and 1716, and 25 % slower on
+// 680.)  Other modes: a warp per tile, so that its accesses are whole lines; the last tile moves back to end with the row,
+// but with dot products (MD), where a thread's elements are part of the sums' values, its columns past the end repeat the
+// last.
 template <typename T, int M, int HB, bool MZ, bool MD, bool RO>
 __device__ __forceinline__ DotAcc srs_tiles(const SrsItem<T> &it, const ItemHops<T> &hops, const T *__restrict__ xs) {
   using TG = TileGeom<T>;
   constexpr int C = TG::C;
+  constexpr bool linear = M == kVec;
   DotAcc acc;
   dot_init(acc);
-  const int ngr = (it.nrows + TG::R - 1) / TG::R, ncb = (it.Nd + TG::W - 1) / TG::W, lane = threadIdx.x & 31;
-  const bool linear = M == kVec && (sizeof(T) == 8 || MD || 8 * ncb * TG::W > 9 * it.Nd);
-  const int per = linear ? it.Nd / C : ncb;
+  const int ngr = (it.nrows + TG::R - 1) / TG::R, per = linear ? it.Nd / C : (it.Nd + TG::W - 1) / TG::W;
 #pragma unroll 1
   for (int unit = linear ? threadIdx.x : threadIdx.x >> 5; unit < ngr * per; unit += linear ? kMvBlock : kMvBlock / 32) {
-    const int g = unit / per, q = unit - g * per;
-    const int cb = linear ? 0 : q * TG::W, want = linear ? q * C : M == kVec ? cb + C * lane : (MD ? cb : min(cb, it.Nd - TG::W)) + lane;
-    srs_tile<T, M, HB, MZ, MD, RO>(it, hops, g * TG::R, cb, M == kVec ? min(want, it.Nd - C) : want, want < it.Nd,
-                               xs, acc);
+    const int g = unit / per, q = unit - g * per, cb = linear ? 0 : q * TG::W;
+    const int c0 = linear ? q * C : (MD ? cb : min(cb, it.Nd - TG::W)) + (threadIdx.x & 31);
+    srs_tile<T, M, HB, MZ, MD, RO>(it, hops, g * TG::R, cb, c0, c0 < it.Nd, xs, acc);
   }
   return acc;
 }
