@@ -282,3 +282,22 @@ def test_item_sizes_against_oracle(elems):
     r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=900,
                        env=dict(os.environ, EDGPU_SRS_ITEM_ELEMS=str(elems), PYTHONPATH=root))
     assert r.returncode == 0 and "ok" in r.stdout, r.stderr[-3000:]
+
+
+# an infinite element reaches its own place and those that H binds it to; every other element keeps its value (rows of
+# 5005 states: two passes)
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_infinite_element_stays_on_its_bonds(ed, precision):
+    params, data = models.random_siam(6, 14)
+    ham = ed.Hamiltonian(ed.Params(params), data, storage="SRS", precision=precision)
+    ham.set_limits(0, 0)
+    n = ham.storage.fill(4, 6)
+    v = np.random.default_rng(2).standard_normal(n)
+    for i in (0, 5, n // 2 + 1234, n - 7):
+        e, z, inf = np.zeros(n), v.copy(), v.copy()
+        e[i], z[i], inf[i] = 1.0, 0.0, np.inf
+        bound = ham.storage.av(e) != 0
+        bound[i] = True
+        w, w0 = ham.storage.av(inf), ham.storage.av(z)
+        assert np.array_equal(w[~bound], w0[~bound])
+    ham.close()
