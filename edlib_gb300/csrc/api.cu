@@ -279,6 +279,7 @@ int edgpu_spmv(edgpu_model *m, int storage, int nup, int ndn, const void *x, voi
                                   : row_item(s->dim * nvec, 64);
       v.per = (int)(((s->storage == kSRS ? s->up_rows : s->dim) + v.rows - 1) / v.rows);
       if ((long long)v.per * nvec > INT_MAX) throw ApiError(EDGPU_ERR_ARG, "too many vectors for one call");
+      sh.short_rows = s->storage == kSRS && s->dn_rows < kSrsLongRow;
       launch_mv_vectors<T>(v, sh, st);
       CK(cudaGetLastError());
     };

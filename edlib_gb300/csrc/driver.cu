@@ -400,6 +400,7 @@ void ensure_ff(edgpu_model *m, Sector *s) {
   o.up_rp = d.up_rp;
   o.up_col = d.up_col;
   o.up_val = up->vff.as<ffloat>();
+  o.up_kmax = d.up_kmax;
   o.dn_len = d.dn_len;
   o.dn_ell_col = d.dn_ell_col;
   o.dn_ell_val = dn->ell_vff.as<ffloat>();
@@ -467,6 +468,7 @@ Sector *get_sector(edgpu_model *m, int storage, int nup, int ndn) {
     s->op64.up_col = s->op32.up_col = up->col.as<int>();
     s->op64.up_val = up->v64.as<double>();
     s->op32.up_val = up->v32.as<float>();
+    s->op64.up_kmax = s->op32.up_kmax = up->kmax;
     s->op64.dn_len = s->op32.dn_len = dn->len.as<int>();
     s->op64.dn_ell_col = s->op32.dn_ell_col = dn->ell_col.as<int>();
     s->op64.dn_ell_val = dn->ell_v64.as<double>();
@@ -498,7 +500,6 @@ Sector *get_sector(edgpu_model *m, int storage, int nup, int ndn) {
     }
     s->srs_rows = srs_item_rows(s->up_rows, s->dn_rows);
     s->nitems = (s->up_rows + s->srs_rows - 1) / s->srs_rows;
-    s->up_kmax = up->kmax;
   } else {
     s->srs_rows = row_item(s->dim, 128);  // an eigen-solver step has many sectors
     s->nitems = (int)((s->dim + s->srs_rows - 1) / s->srs_rows);
@@ -566,7 +567,7 @@ MvShape mv_shape(const Sector &s, bool lz) {
     } else {
       sh.other = 1;
       sh.xs_elems = (int)(s.dn_rows < kSrsVeryLong ? rows * s.dn_rows : std::min(rows * s.dn_rows, cap));
-      sh.hop_elems = item_hop_room(item, s.dn_rows, s.up_kmax);
+      sh.hop_elems = item_hop_room(item, s.dn_rows, s.op64.up_kmax);
     }
   }
   return sh;

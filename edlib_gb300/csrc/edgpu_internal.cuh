@@ -206,6 +206,7 @@ struct SectorOp {
   // spin-resolved Kronecker pieces (SpinResolvedStorage.h:622-638)
   const int *up_rp, *up_col;
   const T *up_val;
+  int up_kmax;        // up hops of the longest row
   // the down-spin matrix k-major ("ELL"): entry k of row d at [k * dn_ld + d], row lengths dn_len[d];
   // dn_ld = dn_rows rounded up to 4, so 4 consecutive rows load as one 16-byte vector
   const int *dn_len, *dn_ell_col;

@@ -333,6 +333,7 @@ struct MvShape {
   int hop_elems = 0;  // up hops of a tiled item
   int long_places = 0;  // rows or columns of the largest two-pass sector (0: none)
   int other = 0;        // some sector is not a two-pass one
+  int short_rows = 0;   // one sector, of short rows
   int plain = 0;
   int mb = 2;         // resident blocks per SM of the eigen-step operator kernel: 2 or 3 (plain launches: 3)
 };

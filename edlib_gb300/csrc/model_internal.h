@@ -123,7 +123,6 @@ struct Sector {
   DBuf dopff;
   int srs_rows = 1, nitems = 1;        // items of products and eigen-solver steps
   int lz_rows = 1, lz_nitems = 1;      // items of recurrences (lz_item_rows)
-  int up_kmax = 0;                     // SRS: up hops of the longest row
   bool complete = false;  // the tables are known to be built (edgpu_spmv runs on streams of its callers)
   template <typename T> const SectorOp<T> &op() const;
   template <typename T> const SectorOp<T> *dop() const;

@@ -180,6 +180,7 @@ struct SrsItem {
   const LzTask<T> *lz;       // the recurrence it belongs to (with dot)
   T c;                       // y = H x + c z
   int Nd, ld, u0, nrows, vloc, skip;
+  int together;              // short rows: a few rows of a column per thread (srs_short)
 };
 
 template <typename T>
@@ -207,6 +208,7 @@ __device__ __forceinline__ void fetch_item(SrsItem<T> &d, const SectorOp<T> *opp
   d.u0 = u0;
   d.nrows = min(srs_rows, op.up_rows - u0);
   d.vloc = op.nW != 0 || op.nV != 0;
+  d.together = sizeof(T) == 4 ? op.up_kmax <= 16 : d.vloc;
   d.skip = srs_two_pass(op.up_rows, Nd);  // k_srs_long's
 }
 
@@ -661,9 +663,12 @@ __device__ __noinline__ DotAcc srs_longrow(const SrsItem<T> &it, const T *__rest
 
 // SRS item of short rows (below kSrsLongRow states), staged like a tile's (stage_interleaved, slots in column order):
 // a thread takes one column of RI rows at a time, so that rows shorter than a warp keep every thread busy and each
-// down-hop entry, loaded once, serves RI rows.  Per element the sums of the tiles, in the reference's order.
-// 12-orbital impurity, rows of 66 states, FP32: 21 ps per state, rows of 12: 25 (20 and 24 one element per
-// thread, the CSR entry by entry; 33 and 53 that way in a block of two per SM).
+// down-hop entry, loaded once, serves RI rows; or (srs_flat) one element at a time.  Per element the sums of the tiles, in
+// the reference's order.  Columns of rows for FP32 vectors (32 of them, 12-orbital impurity, rows of 66 states 41 us, one
+// element at a time 47; 14-site ring, rows of 91: 67 and 72) but not with many up hops per row, which nothing is shared of
+// (16-site square cluster, 8 vectors, rows of 16 states: 120 and 87 us, 120 states: 571 and 561); 8-byte types, bound by
+// arithmetic, one element at a time (rows of 66 states 95 and 84 us) but with interaction terms, whose chains of loads run
+// side by side for the rows (G of the 8-orbital Kanamori impurity 4.46 and 4.67 ms).
 template <typename T, bool MZ>
 __device__ __noinline__ void srs_short(const SrsItem<T> &it, const ItemHops<T> &hops, bool near, const T *__restrict__ xs) {
   constexpr int RI = Lanes<T>::C;
@@ -751,9 +756,9 @@ __device__ __noinline__ void srs_short(const SrsItem<T> &it, const ItemHops<T> &
   }
 }
 
-// The same with dot products: a thread takes one element at a time, e = threadIdx.x, + kMvBlock, ... over the item, which
-// is part of the value of <x, y>.
-template <typename T, bool MZ>
+// A thread takes one element at a time, e = threadIdx.x, + kMvBlock, ... over the item, which with dot products (MD) is part
+// of the value of <x, y>.
+template <typename T, bool MZ, bool MD>
 __device__ __noinline__ DotAcc srs_flat(const SrsItem<T> &it, const ItemHops<T> &hops, bool near, const T *__restrict__ xs) {
   constexpr int RI = Lanes<T>::C;
   const SectorOp<T> &op = *it.op;
@@ -787,7 +792,7 @@ __device__ __noinline__ DotAcc srs_flat(const SrsItem<T> &it, const ItemHops<T> 
     }
     if (it.vloc) a = srs_vloc<T, 1, 1>(it.op, it.u0 + r, d, it.x, RowPart<T, 1>{{a}}).v[0];
     it.y[e] = renorm(a);
-    dot_add(acc, xv, a);
+    if (MD && it.dot) dot_add(acc, xv, a);
     r += rs;
     d += ds;
     if (d >= Nd) d -= Nd, ++r;
@@ -1014,7 +1019,7 @@ __global__ void __launch_bounds__(kMvBlock, MB) k_srs_mv(Src src, int nitems, in
       else if (!whole) acc = srs_tiles<T, kOdd, HB, MZ, MD, RO>(it, hops, xs);
       else acc = srs_tiles_off<T, MZ, MD, RO>(it, hops, xs);
     } else if (small) {
-      if constexpr (MD) acc = srs_flat<T, MZ>(it, hops, near, xs);
+      if (MD || !it.together) acc = srs_flat<T, MZ, MD>(it, hops, near, xs);
       else srs_short<T, MZ>(it, hops, near, xs);
     } else {
       acc = srs_longrow<T, MZ, MD>(it, nel <= xs_cap ? xs : it.xi);
@@ -1300,6 +1305,10 @@ void launch_mv_vectors(const Sector_mv<T> &v, MvShape sh, cudaStream_t st) {
   const VecSource<T> src{v.op, v.x, v.y, v.ld, v.rows, v.per, v.accumulate};
   const int n = v.per * v.nvec;
   if (sh.storage != kSRS) launch_rows<T>(sh.storage, src, n, st);
+  // short rows wait on memory, not on L1: three blocks per SM for every type (16-site square cluster, FP32 rows of 16 states
+  // 107 us with two, 87 with three)
+  else if (sh.short_rows && v.accumulate) launch_srs<T, VecSource<T>, true, false, 1, 3>(src, n, sh, st);
+  else if (sh.short_rows) launch_srs<T, VecSource<T>, false, false, 1, 3>(src, n, sh, st);
   else if (v.accumulate) launch_srs<T, VecSource<T>, true, false, 1, kMvBlocks<T>>(src, n, sh, st);
   else launch_srs<T, VecSource<T>, false, false, kPlainHB<T>, kMvBlocks<T>>(src, n, sh, st);
 }

@@ -301,3 +301,13 @@ def test_infinite_element_stays_on_its_bonds(ed, precision):
         w, w0 = ham.storage.av(inf), ham.storage.av(z)
         assert np.array_equal(w[~bound], w0[~bound])
     ham.close()
+
+
+# short rows with many up hops (one element at a time; more hops per item than its shared memory holds) and few
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_short_rows_with_many_up_hops_against_oracle(ed, precision):
+    t = models.square_hopping(4, 3, 1.0, -0.3)
+    check_products(ed, {"NSITES": 12, "NSPINS": 2}, models.hubbard(t, 4.0, 2.0), "HUBBARD", "SRS", [(6, 1), (6, 2), (2, 10)],
+                   precision)
+    params, data = models.random_siam(3, 11)
+    check_products(ed, params, data, "SIAM", "SRS", [(6, 1), (6, 2), (7, 0)], precision)
