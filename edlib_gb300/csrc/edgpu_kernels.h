@@ -24,7 +24,7 @@ void note_launch(long long n = 1);
 
 // A launch that may start while the kernel before it in the stream still runs (programmatic dependent launch); the
 // kernel calls pdl_enter (edgpu_internal.cuh) before it reads anything, so only the launch itself and the set-up of
-// shared memory overlap.  The recurrences' steps of two small kernels gain by it; the eigen-solver's do not (its
+// shared memory overlap.  The recurrences' steps of three or four small kernels gain by it; the eigen-solver's do not (its
 // Gram-Schmidt passes' stages and the operator's L1 want the same memory: 12-orbital solve 5 % slower, 8-site ring 1 %
 // faster).
 template <class... P, class... A>

@@ -6,18 +6,22 @@
 //            accumulated per element in the reference order (diagonal, down hops, up hops, interaction).
 //            A work item is a group of up-rows; its rows of X are staged in shared memory, so that the H_dn
 //            gather reads shared memory, and the H_up term reads whole rows of X (coalesced in d).  Rows of
-//            kSrsLongRow to kSrsVeryLong - 1 states in tiles of 4 rows x 32 C columns per warp over row-interleaved
-//            shared memory (srs_tile); longer rows one at a time (srs_longrow); shorter ones a
-//            column of a few rows per thread (srs_short).
-//            The off-diagonal interaction (H_loc): terms between the spins from one-spin hop tables (products of
-//            an up and a down hop), the others matrix-free from the transition list.
+//            kSrsLongRow to kSrsVeryLong - 1 states in tiles of 4 rows over row-interleaved shared memory (srs_tile);
+//            longer rows one at a time (srs_longrow) or, in sectors of many of them, in two passes (k_srs_long);
+//            shorter ones a column of a few rows or one element per thread (srs_short, srs_flat).
+//            The off-diagonal interaction (H_loc): from tables of its terms' one-spin halves, or matrix-free from the
+//            transition list.
 //            Element types: FP32, FP64, and float-float pairs (the mixed mode's recurrences).
-// * CRS   -- CRSStorage::av (include/edlib/CRSStorage.h:57-64): four lanes per row.
+// * CRS   -- CRSStorage::av (include/edlib/CRSStorage.h:57-64): a thread per row.
 // * SOCRS -- SOCRSStorage::av (include/edlib/SOCRSStorage.h:46-87): matrix-free; each row re-derives its
 //            state from the combinadic tables, tests every transition by its masks, ranks the target with ninv
-//            and takes the fermion sign from one popc; nothing but the tables is stored.  Eight lanes per row.
-// Every kernel is instantiated per storage (a launch covers one storage) and optionally emits <x, y>
-// per item (FP64 / float-float accumulation, fixed order).
+//            and takes the fermion sign from one popc; nothing but the tables is stored.  A thread per row.
+// Every kernel is instantiated per storage (a launch covers one storage); the recurrences' emit <x, y> per item (FP64 /
+// float-float accumulation, fixed order).
+//
+// The order of every sum is part of the values.  Eigen-solves stop and restart on them, and two kinds of results magnify a
+// last bit: a continued fraction that has not converged (of a state that is not the lowest of its neighbouring sectors;
+// by up to 1e11), and the last, near-degenerate pairs of a solve.
 
 #pragma once
 #include "edgpu_kernels.h"
@@ -40,7 +44,7 @@ __device__ __forceinline__ ffloat madd(ffloat a, ffloat b, ffloat c) { return c 
 
 template <typename T>
 __device__ __forceinline__ T transitions_term(const SectorOp<T> &op, state_t s, const Transition *L, const T *vals, int nL,
-                                              const T *__restrict__ x, T acc) {
+                                              const T *x, T acc) {
   for (int q = 0; q < nL; ++q) {
     if (!trans_valid(L[q], s, op.ip)) continue;
     int sign;
