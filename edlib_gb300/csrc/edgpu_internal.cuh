@@ -489,25 +489,6 @@ __device__ __forceinline__ void pdl_enter() {
   asm volatile("griddepcontrol.wait;\n griddepcontrol.launch_dependents;\n" ::: "memory");
 }
 
-// The last of n blocks to finish a part (each called once by a whole block, after thread 0 wrote part[own]) gets the
-// sum of all parts, in a fixed order, in thread 0 and true; the count is zero again then.  No block waits for another.
-template <int BLOCK>
-__device__ inline bool last_block_sum(const double *part, int n, int *count, double *red, double &sum) {
-  __shared__ int last;
-  if (threadIdx.x == 0) {
-    __threadfence();
-    last = atomicAdd(count, 1) == n - 1;
-  }
-  __syncthreads();
-  if (!last) return false;  // uniform over the block
-  __threadfence();
-  double s = 0.0;
-  for (int k = threadIdx.x; k < n; k += blockDim.x) s += __ldcg(part + k);
-  sum = block_sum<BLOCK>(s, red);
-  if (threadIdx.x == 0) *count = 0;
-  return true;
-}
-
 // ---------------------------------------------------------------- continued fraction
 __device__ inline double2 cmul(double2 a, double2 b) { return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
 __device__ inline double2 cdiv(double2 a, double2 b) {

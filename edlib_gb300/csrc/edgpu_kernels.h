@@ -237,8 +237,8 @@ struct LzTask {
   double *beta;       // [nlanc + 1]
   double *part_a;     // [nitems]
   double *part_b;     // [nitems]
-  double *scal;       // [0] alf, [1] bet
-  int *state;         // [0] done, [1] nlanc, [2] items whose <v, w> is done in this step, [3] of the alpha pass
+  double *scal;       // [0] bet
+  int *state;         // [0] 0, or the step (from 1) that finished it, [1] nlanc
   int nlanc_max;
   int mv_rows;        // rows per item and first item of the product, where it has items of its own (LzBatch::split)
   int mv_begin;

@@ -155,12 +155,12 @@ void run_lanczos_ff(edgpu_model *m, std::vector<LzJob<double> *> &jobs, int nlan
     J.beta = DBuf(c->alloc, sizeof(double) * (nlanc + 1));
     J.part_a = DBuf(c->alloc, sizeof(double) * s.lz_nitems);
     J.part_b = DBuf(c->alloc, sizeof(double) * s.lz_nitems);
-    J.scal = DBuf(c->alloc, sizeof(double) * 2);
-    J.state = DBuf(c->alloc, sizeof(int) * 4);
+    J.scal = DBuf(c->alloc, sizeof(double));
+    J.state = DBuf(c->alloc, sizeof(int) * 2);
     CK(cudaMemsetAsync(J.alpha.p, 0, sizeof(double) * nlanc, c->stream));
     CK(cudaMemsetAsync(J.beta.p, 0, sizeof(double) * (nlanc + 1), c->stream));
-    CK(cudaMemsetAsync(J.scal.p, 0, sizeof(double) * 2, c->stream));
-    CK(cudaMemsetAsync(J.state.p, 0, sizeof(int) * 4, c->stream));
+    CK(cudaMemsetAsync(J.scal.p, 0, sizeof(double), c->stream));
+    CK(cudaMemsetAsync(J.state.p, 0, sizeof(int) * 2, c->stream));
     LzTask<ffloat> &t = tasks[q];
     t.op = s.dop<ffloat>();
     t.srs_rows = s.lz_rows;
@@ -214,12 +214,12 @@ void run_lanczos(edgpu_model *m, std::vector<LzJob<T> *> &jobs, int nlanc, bool 
     J.beta = DBuf(c->alloc, sizeof(double) * (nlanc + 1));
     J.part_a = DBuf(c->alloc, sizeof(double) * s.lz_nitems);
     J.part_b = DBuf(c->alloc, sizeof(double) * s.lz_nitems);
-    J.scal = DBuf(c->alloc, sizeof(double) * 2);
-    J.state = DBuf(c->alloc, sizeof(int) * 4);
+    J.scal = DBuf(c->alloc, sizeof(double));
+    J.state = DBuf(c->alloc, sizeof(int) * 2);
     CK(cudaMemsetAsync(J.alpha.p, 0, sizeof(double) * nlanc, c->stream));
     CK(cudaMemsetAsync(J.beta.p, 0, sizeof(double) * (nlanc + 1), c->stream));
-    CK(cudaMemsetAsync(J.scal.p, 0, sizeof(double) * 2, c->stream));
-    CK(cudaMemsetAsync(J.state.p, 0, sizeof(int) * 4, c->stream));
+    CK(cudaMemsetAsync(J.scal.p, 0, sizeof(double), c->stream));
+    CK(cudaMemsetAsync(J.state.p, 0, sizeof(int) * 2, c->stream));
     LzTask<T> &t = tasks[q];
     t.op = s.dop<T>();
     t.srs_rows = s.lz_rows;

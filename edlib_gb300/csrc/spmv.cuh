@@ -181,7 +181,6 @@ struct SrsItem {
   const int *len, *urp;      // urp: from the item's first row on
   const Hop<T> *uh;
   double *dot;               // the item's part of <x, y>, or null
-  const LzTask<T> *lz;       // the recurrence it belongs to (with dot)
   T c;                       // y = H x + c z
   int Nd, ld, u0, nrows, vloc, skip;
   int together;              // short rows: a few rows of a column per thread (srs_short)
@@ -205,7 +204,6 @@ __device__ __forceinline__ void fetch_item(SrsItem<T> &d, const SectorOp<T> *opp
   d.urp = op.up_rp + u0;
   d.uh = op.up_hop;
   d.dot = lz ? lz->part_a + li : nullptr;
-  d.lz = lz;
   d.c = c;
   d.Nd = Nd;
   d.ld = op.dn_ld;
@@ -867,13 +865,11 @@ __device__ __forceinline__ void mv_item(const SectorOp<T> *opp, int rows, long l
   }
 }
 
-// <x, y> of an item into its recurrence's parts; the block that finishes the task's last item sums them: alf.
-template <typename T, int NT>
-__device__ __forceinline__ void emit_dot(const LzTask<T> &t, DotAcc &acc, double *dst, double *red) {
+// <x, y> of an item into its recurrence's parts
+template <int NT>
+__device__ __forceinline__ void emit_dot(DotAcc &acc, double *dst, double *red) {
   const double s = block_sum<NT>(dot_value(acc), red);
   if (threadIdx.x == 0) *dst = s;
-  double alf;
-  if (last_block_sum<NT>(t.part_a, t.nitems, t.state + 2, red, alf) && threadIdx.x == 0) t.scal[0] = alf;
 }
 
 // ---------------------------------------------------------------- where an operator launch's items come from
@@ -928,7 +924,7 @@ struct LzSource {
     const LzTask<T> &t = tasks[item_task[it]];
     if (t.state[0]) return false;
     f(t.op, SPLIT ? t.mv_rows : t.srs_rows, it - (SPLIT ? t.mv_begin : t.item_begin), t.buf[iter % 3], t.buf[(iter + 1) % 3],
-      iter == 0 ? nullptr : t.buf[(iter + 2) % 3], (T)(-t.scal[1]), SPLIT ? (const LzTask<T> *)nullptr : &t);
+      iter == 0 ? nullptr : t.buf[(iter + 2) % 3], (T)(-t.scal[0]), SPLIT ? (const LzTask<T> *)nullptr : &t);
     return true;
   }
 };
@@ -1028,7 +1024,7 @@ __global__ void __launch_bounds__(kMvBlock, MB) k_srs_mv(Src src, int nitems, in
     } else {
       acc = srs_longrow<T, MZ, MD>(it, nel <= xs_cap ? xs : it.xi);
     }
-    if (MD && it.dot) emit_dot<T, kMvBlock>(*it.lz, acc, it.dot, red);
+    if (MD && it.dot) emit_dot<kMvBlock>(acc, it.dot, red);
     __syncthreads();  // xs and items[p] are free, items[p ^ 1] is there
   }
 }
@@ -1206,7 +1202,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_srs_long(Src src, int nitems)
           }
         }
       }
-      if (MD && it.dot) emit_dot<T, NT>(*it.lz, acc, it.dot, red);
+      if (MD && it.dot) emit_dot<NT>(acc, it.dot, red);
     }
   }
 }
