@@ -204,8 +204,14 @@ void run_lanczos(edgpu_model *m, std::vector<LzJob<T> *> &jobs, int nlanc, bool 
   }
   std::vector<LzTask<T>> tasks(jobs.size());
   std::vector<int> item_task, mv_item_task;
-  bool split = true;  // only rows that are short or stored row by row: items of 2048 elements, a handful per recurrence
-  for (auto *J : jobs) split = split && (J->s->storage != kSRS || J->s->dn_rows < kSrsLongRow);
+  // only rows that are short or stored row by row: items of 2048 elements, a handful per recurrence; where the product's
+  // own items are no smaller (SRS), its <v, w> needs no pass of its own
+  bool split = true, smaller = false;
+  for (auto *J : jobs) {
+    split = split && (J->s->storage != kSRS || J->s->dn_rows < kSrsLongRow);
+    smaller = smaller || J->s->storage != kSRS || J->s->srs_rows < J->s->lz_rows;
+  }
+  split = split && smaller;
   MvShape shape{jobs[0]->s->storage, 0};
   for (size_t q = 0; q < jobs.size(); ++q) {
     LzJob<T> &J = *jobs[q];

@@ -1324,6 +1324,15 @@ void launch_lz_mv(const LzBatch<T> &b, int it, bool early, MvShape sh, cudaStrea
     }
   }
   const LzSource<T, false> src{b.tasks, b.item_task, it};
+  if constexpr (sizeof(T) == 8) {
+    // few items: no more blocks per SM than registers for two rounds of up hops in flight allow (G of the 11-orbital
+    // impurity, 99 items, float-float 7.6 -> 6.1 ms, FP64 8.8 -> 8.3); FP64, bound by arithmetic, one (198 items of the same
+    // sizes: 11.9 ms with either)
+    if (b.nitems <= (std::is_same<T, ffloat>::value ? 2 : 1) * kSms) {
+      launch_srs<T, LzSource<T, false>, true, true, 2, 2>(src, b.nitems, sh, st, early);
+      return;
+    }
+  }
   launch_srs<T, LzSource<T, false>, true, true, 1, kMvBlocks<T>>(src, b.nitems, sh, st, early);
 }
 

@@ -311,3 +311,26 @@ def test_short_rows_with_many_up_hops_against_oracle(ed, precision):
                    precision)
     params, data = models.random_siam(3, 11)
     check_products(ed, params, data, "SIAM", "SRS", [(6, 1), (6, 2), (7, 0)], precision)
+
+
+# float-float and FP64 recurrences one at a time (few items: launches that start early, two blocks per SM) and all in one
+# batch: each path adds in the same order.  Items of one recurrence, and of the batch of four kept states' sixteen: 10
+# orbitals 7 and 112, 11 29 and 400 (tiles, rows of 210 to 462 states); 9 orbitals 6 to 8 and 112 (rows of 126).
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("ns", [9, 10, 11])
+def test_recurrences_independent_of_their_batch(ed, ns, precision):
+    params, data = models.random_siam(21, ns - 1)
+    params.update({"arpack.NEV": 4, "arpack.SECTOR": 1, "lanc.BETA": 2.0, "lanc.NOMEGA": 16, "lanc.NLANC": 60})
+    data["sectors/values"] = np.array([[ns // 2, ns // 2]], dtype=np.float64)
+    p = ed.Params(params)
+    ham = ed.Hamiltonian(p, data, storage="SRS", precision=precision)
+    ham.set_limits(0, 0)
+    ham.diag()
+    G = []
+    for ham.max_batch in (0, 1, 3):
+        g = ed.GreensFunction(p, ham)
+        g.compute()
+        G.append(g.G.copy())
+    ham.close()
+    assert np.all(np.isfinite(G[0])) and np.abs(G[0]).max() > 0
+    assert np.array_equal(G[0], G[1]) and np.array_equal(G[0], G[2])
