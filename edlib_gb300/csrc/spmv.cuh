@@ -665,11 +665,11 @@ __device__ __noinline__ DotAcc srs_longrow(const SrsItem<T> &it, const T *__rest
 
 // SRS item of short rows (below kSrsLongRow states), staged like a tile's (stage_interleaved, slots in column order):
 // a thread takes one column of RI rows at a time, so that rows shorter than a warp keep every thread busy and each
-// down-hop entry, loaded once, serves RI rows; or (srs_flat) one element at a time.  Per element the sums of the tiles, in
-// the reference's order.  Columns of rows for FP32 vectors (32 of them, 12-orbital impurity, rows of 66 states 41 us, one
-// element at a time 47; 14-site ring, rows of 91: 67 and 72) but not with many up hops per row, which nothing is shared of
-// (16-site square cluster, 8 vectors, rows of 16 states: 120 and 87 us, 120 states: 571 and 561); 8-byte types, bound by
-// arithmetic, one element at a time (rows of 66 states 95 and 84 us) but with interaction terms, whose chains of loads run
+// down-hop entry, loaded once, serves RI rows; or (srs_flat, rows as they are) one element at a time.  Per element the sums
+// of the tiles, in the reference's order.  Columns of rows for FP32 vectors of few up hops per row (32 vectors, 12-orbital
+// impurity, rows of 66 states 39 us, one element at a time 41; but 14-site ring, rows of 91: 160 and 147), which nothing is
+// shared of where they are many (16-site square cluster, 8 vectors, rows of 16 states: 121 and 66 us); 8-byte types, bound by
+// arithmetic, one element at a time (rows of 66 states 95 and 83 us) but with interaction terms, whose chains of loads run
 // side by side for the rows (G of the 8-orbital Kanamori impurity 4.46 and 4.67 ms).
 template <typename T, bool MZ>
 __device__ __noinline__ void srs_short(const SrsItem<T> &it, const ItemHops<T> &hops, bool near, const T *__restrict__ xs) {
@@ -759,10 +759,10 @@ __device__ __noinline__ void srs_short(const SrsItem<T> &it, const ItemHops<T> &
 }
 
 // A thread takes one element at a time, e = threadIdx.x, + kMvBlock, ... over the item, which with dot products (MD) is part
-// of the value of <x, y>.
+// of the value of <x, y>.  The item's rows are copied as they are: interleaved like the others' they came through registers
+// and cost twice the shared-memory wavefronts (G of the 9-orbital impurity, FP64, 4.43 -> 4.19 ms).
 template <typename T, bool MZ, bool MD>
 __device__ __noinline__ DotAcc srs_flat(const SrsItem<T> &it, const ItemHops<T> &hops, bool near, const T *__restrict__ xs) {
-  constexpr int RI = Lanes<T>::C;
   const SectorOp<T> &op = *it.op;
   const int Nd = it.Nd, ld = it.ld, n = it.nrows * Nd, first = ldg_t(it.urp);
   const int *__restrict__ ecol = op.dn_ell_col;
@@ -772,25 +772,27 @@ __device__ __noinline__ DotAcc srs_flat(const SrsItem<T> &it, const ItemHops<T> 
   int r = threadIdx.x / Nd, d = threadIdx.x - r * Nd;
   const int rs = kMvBlock / Nd, ds = kMvBlock - rs * Nd;
   for (int e = threadIdx.x; e < n; e += kMvBlock) {
-    const T *__restrict__ xg = xs + (r / RI) * Nd * RI + r % RI;
-    const T xv = xg[d * RI];
+    const T *__restrict__ xg = xs + r * Nd;
+    const T xv = xg[d];
     T a = mul_rn(ldg_t(it.dg + e), xv);
     if (MZ && it.z) a = madd(it.c, it.z[e], a);
     const int kk = ldg_t(it.len + d);
 #pragma unroll 4
-    for (int k = 0; k < kk; ++k) a = madd(ldg_t(eval + k * ld + d), xg[ldg_t(ecol + k * ld + d) * RI], a);
+    for (int k = 0; k < kk; ++k) a = madd(ldg_t(eval + k * ld + d), xg[ldg_t(ecol + k * ld + d)], a);
     const int k0 = ldg_t(it.urp + r), nh = ldg_t(it.urp + r + 1) - k0;
     const T *xd = it.x + d;
+    if (near) {
 #pragma unroll 4
-    for (int h = 0; h < nh; ++h) {
-      Hop<T> hp;
-      if (near) {
-        hp = hops.hop[k0 - first + h];
-      } else {
-        hp = ldg_hop(it.uh + k0 + h);
-        hp.c *= Nd;
+      for (int h = 0; h < nh; ++h) {
+        const Hop<T> hp = hops.hop[k0 - first + h];
+        a = madd(hp.v, xd[hp.c], a);
       }
-      a = madd(hp.v, xd[hp.c], a);
+    } else {
+#pragma unroll 8
+      for (int h = 0; h < nh; ++h) {
+        const Hop<T> hp = ldg_hop(it.uh + k0 + h);
+        a = madd(hp.v, xd[hp.c * Nd], a);
+      }
     }
     if (it.vloc) a = srs_vloc<T, 1, 1>(it.op, it.u0 + r, d, it.x, RowPart<T, 1>{{a}}).v[0];
     it.y[e] = renorm(a);
@@ -978,7 +980,7 @@ __global__ void __launch_bounds__(kMvBlock, MB) k_srs_mv(Src src, int nitems, in
       continue;
     }
     const int Nd = it.Nd;
-    const bool small = Nd < kSrsLongRow;
+    const bool small = Nd < kSrsLongRow, flat = small && (MD || !it.together);
     bool tile = Nd >= kSrsLongRow && Nd < kSrsVeryLong;
     // 16-byte accesses: rows of whole 16-byte pieces on aligned bases
     const bool whole = (Nd * sizeof(T)) % 16 == 0;
@@ -1005,13 +1007,13 @@ __global__ void __launch_bounds__(kMvBlock, MB) k_srs_mv(Src src, int nitems, in
       if (vec) stage_interleaved<T, kVec, RO>(xs, it.xi, it.nrows, Nd);
       else if (!whole) stage_interleaved<T, kOdd, RO>(xs, it.xi, it.nrows, Nd);
       else stage_interleaved<T, kOff, RO>(xs, it.xi, it.nrows, Nd);
-    } else if (small) {
+    } else if (small && !flat) {
       stage_interleaved<T, kOdd, RO>(xs, it.xi, it.nrows, Nd);
     } else if (nel <= xs_cap) {
       stage_async(xs, it.xi, nel);
     }
     if (threadIdx.x == kMvBlock - 32) fetch(i + gridDim.x, items[p ^ 1]);  // the next item's description
-    if (!tile && !small) cp_async_wait_all();
+    if (!tile && (!small || flat)) cp_async_wait_all();
     __syncthreads();
     DotAcc acc{};
     if (tile) {
@@ -1019,7 +1021,7 @@ __global__ void __launch_bounds__(kMvBlock, MB) k_srs_mv(Src src, int nitems, in
       else if (!whole) acc = srs_tiles<T, kOdd, HB, MZ, MD, RO>(it, hops, xs);
       else acc = srs_tiles_off<T, MZ, MD, RO>(it, hops, xs);
     } else if (small) {
-      if (MD || !it.together) acc = srs_flat<T, MZ, MD>(it, hops, near, xs);
+      if (flat) acc = srs_flat<T, MZ, MD>(it, hops, near, xs);
       else srs_short<T, MZ>(it, hops, near, xs);
     } else {
       acc = srs_longrow<T, MZ, MD>(it, nel <= xs_cap ? xs : it.xi);
@@ -1306,7 +1308,7 @@ void launch_mv_vectors(const Sector_mv<T> &v, MvShape sh, cudaStream_t st) {
   const int n = v.per * v.nvec;
   if (sh.storage != kSRS) launch_rows<T>(sh.storage, src, n, st);
   // short rows wait on memory, not on L1: three blocks per SM for every type (16-site square cluster, FP32 rows of 16 states
-  // 107 us with two, 87 with three)
+  // 82 us with two, 66 with three)
   else if (sh.short_rows && v.accumulate) launch_srs<T, VecSource<T>, true, false, 1, 3>(src, n, sh, st);
   else if (sh.short_rows) launch_srs<T, VecSource<T>, false, false, 1, 3>(src, n, sh, st);
   else if (v.accumulate) launch_srs<T, VecSource<T>, true, false, 1, kMvBlocks<T>>(src, n, sh, st);
